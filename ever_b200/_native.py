@@ -137,6 +137,7 @@ SIGNATURES = {
                                                        c_p]),
     "ever_camera_event_log_to_reference": (ctypes.c_int, [ctypes.POINTER(EverScene), ctypes.POINTER(EverCamera),
                                                           c_p, c_i32, c_p, c_p, c_i32, c_p]),
+    "ever_depth_hint": (ctypes.c_int, [c_p, c_p, c_p, c_i64, ctypes.POINTER(c_f32), c_f32, c_p, c_p]),
     "ever_ray_order_binned": (ctypes.c_int, [c_p, c_p, c_p, c_i64, c_p, c_sz, c_p, c_p]),
     "ever_batch_order_binned": (ctypes.c_int, [ctypes.POINTER(EverBatch), c_p, c_p, c_p, c_p]),
 }

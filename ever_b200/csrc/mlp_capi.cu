@@ -38,6 +38,26 @@ ever::MlpParams base_params(const EverMlp* m) {
 
 }  // namespace
 
+namespace ever {
+namespace {
+
+// Stopping t from the model's depth output: the offset from the closest point of the ray's
+// line to the centre, times the scale. One pass over the rays (28 B in, 4 B out each); as
+// ten elementwise passes it took longer than the model's inference.
+__global__ void k_depth_hint(const float* __restrict__ pred, const float* __restrict__ rayo,
+                             const float* __restrict__ rayd, int64_t R, float3 c, float scale,
+                             float* __restrict__ out) {
+  const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (r >= R) return;
+  const float dx = rayd[3 * r], dy = rayd[3 * r + 1], dz = rayd[3 * r + 2];
+  const float n = fmaxf(sqrtf((dx * dx + dy * dy) + dz * dz), 1e-30f);
+  const float s = -(((rayo[3 * r] - c.x) * dx + (rayo[3 * r + 1] - c.y) * dy) + (rayo[3 * r + 2] - c.z) * dz) / n;
+  out[r] = (pred[2 * r + 1] * scale + s) / n;
+}
+
+}  // namespace
+}  // namespace ever
+
 extern "C" {
 
 size_t ever_mlp_workspace_bytes(void) { return size_t(ever::kMlpMaxGrid) * (ever::kMlpParams + 1) * sizeof(float); }
@@ -107,6 +127,18 @@ int ever_mlp_adam(const EverMlp* mlp, const float* grads, float* adam_m, float* 
   return cuda_status(ever::launch_mlp_adam(mlp->params, grads, adam_m, adam_v, mlp->w1, mlp->w2, mlp->w3, lr, beta1,
                                            beta2, eps, step, static_cast<cudaStream_t>(stream)),
                      "ever_mlp_adam");
+}
+
+int ever_depth_hint(const float* pred, const float* rayo, const float* rayd, int64_t num_rays, const float* centre,
+                    float scale, float* depth_hint, void* stream) {
+  if (num_rays < 0 || num_rays >= (int64_t(1) << 31))
+    return ever::set_last_error(EVER_ERR_INVALID, "ever_depth_hint: num_rays out of range");
+  if (!centre || (num_rays > 0 && (!pred || !rayo || !rayd || !depth_hint)))
+    return ever::set_last_error(EVER_ERR_INVALID, "ever_depth_hint: null pointer");
+  if (num_rays == 0) return EVER_OK;
+  ever::k_depth_hint<<<unsigned((num_rays + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      pred, rayo, rayd, num_rays, make_float3(centre[0], centre[1], centre[2]), scale, depth_hint);
+  return cuda_status(cudaGetLastError(), "ever_depth_hint");
 }
 
 int ever_ray_order_binned(const float* rayo, const float* rayd, const uint8_t* bins, int64_t num_rays,

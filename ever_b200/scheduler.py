@@ -180,6 +180,17 @@ def depth_from_prediction(pred: torch.Tensor, rayo: torch.Tensor, rayd: torch.Te
                           scale: float = 1.0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """(R,) stopping t guessed by the model (the inverse of cost_targets' depth column): the
     depth hint the tracer's frustum phase takes (tracer.forward(depth_hint=...))."""
+    ts = (pred, rayo, rayd) + (() if out is None else (out,))
+    R = rayo.shape[0]
+    if (all(t.is_cuda and t.device == pred.device and t.dtype == torch.float32 and t.is_contiguous()
+            and not t.requires_grad for t in ts)
+            and rayo.shape == rayd.shape == (R, 3) and pred.shape == (R, 2) and (out is None or out.shape == (R,))):
+        d = torch.empty(R, dtype=torch.float32, device=pred.device) if out is None else out
+        with torch.cuda.device(pred.device):
+            N.check(N.load().ever_depth_hint(N.ptr(pred), N.ptr(rayo), N.ptr(rayd), R,
+                                             (ctypes.c_float * 3)(*[float(v) for v in centre]), float(scale), N.ptr(d),
+                                             ctypes.c_void_p(torch.cuda.current_stream(pred.device).cuda_stream)))
+        return d
     c = torch.tensor(centre, dtype=torch.float32, device=rayo.device)
     n = rayd.norm(dim=1).clamp_min(1e-30)
     s_c = -((rayo - c) * rayd).sum(1) / n

@@ -357,6 +357,12 @@ int ever_mlp_gradients(const EverMlp* mlp, const float* rayo, const float* rayd,
 int ever_mlp_adam(const EverMlp* mlp, const float* grads, float* adam_m, float* adam_v, float lr, float beta1,
                   float beta2, float eps, int32_t step, void* stream);
 
+/* Stopping t per ray from the model's predictions pred (num_rays, 2): the depth hint of
+ * EverTraceArgs. The depth output is the offset along the ray from the point of its line
+ * closest to centre[3], divided by scale. */
+int ever_depth_hint(const float* pred, const float* rayo, const float* rayd, int64_t num_rays, const float* centre,
+                    float scale, float* depth_hint, void* stream);
+
 /* ever_ray_order with cost bins (one byte per ray, 0..3, larger = costlier) on top of the
  * key: costlier bins come first. Same workspace as ever_ray_order. */
 int ever_ray_order_binned(const float* rayo, const float* rayd, const uint8_t* bins, int64_t num_rays,
