@@ -53,12 +53,12 @@ EverTune tune_of(const EverTune* t) {
 }
 
 // Persistent grid: enough resident blocks to fill every SM. Occupancy is bounded by
-// registers: 20 warps per SM for the forward with blocks of 64 or 128 threads, 16 warps
-// with 256 threads; 24 warps for the degree-0 backward, 16 with SH colour.
-int persistent_grid(int block, bool forward, int deg = 0) {
+// registers: 16 warps per SM for the forward with the frustum phase, 20 for gather rounds
+// only (16 with 256 threads); 24 warps for the degree-0 backward, 16 with SH colour.
+int persistent_grid(int block, bool forward, int deg = 0, bool rounds = false) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int warps_per_sm = forward ? (block <= 128 ? 20 : 16) : (deg == 0 ? 24 : 16);
+  const int warps_per_sm = forward ? (rounds && block <= 128 ? 20 : 16) : (deg == 0 ? 24 : 16);
   return std::max(1, sms * std::max(1, warps_per_sm * 32 / block));
 }
 
@@ -181,7 +181,7 @@ int ever_trace_forward_batched(const EverBatch* batch, const float* rayo, const 
   P.max_iters = args->max_iters;
   P.out = *out;
   P.work_counter = batch->counters;
-  P.grid = persistent_grid(tn.block, true);
+  P.grid = persistent_grid(tn.block, true, 0, tn.traversal == 2);
   const cudaError_t e = launch_forward_batched(P, deg, tn, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? EVER_OK : set_last_error(EVER_ERR_CUDA, cudaGetErrorString(e));
 }

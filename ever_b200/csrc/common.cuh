@@ -45,6 +45,9 @@ __device__ __forceinline__ float safe_div(float a, float b) {
 __device__ __forceinline__ float safe_exp(float v) { return expf(clampf(v, kMinVal, kLogMax)); }
 __device__ __forceinline__ float sgnf(float x) { return x > 0.f ? 1.f : (x < 0.f ? -1.f : 0.f); }
 
+// 1 / x as safe_div takes it: the denominator's magnitude is kept from kTiny down.
+__device__ __forceinline__ float safe_rcp(float x) { return 1.f / (fabsf(x) < kTiny ? kTiny : x); }
+
 // tukey_power_ladder(x, -0.1), safe-math.slang:246-253
 __device__ __forceinline__ float tukey(float x) {
   const float p = -0.1f;
@@ -83,22 +86,27 @@ struct __align__(16) Record {
 __device__ __forceinline__ float3 dc_colour(float4 r3) { return make_float3(r3.y, r3.z, r3.w); }
 __device__ __forceinline__ float dc_channel(float f0) { return fmaf(kShC0, f0, 0.5f); }
 
+// One BVH node, 64 B: each child is a 32-byte half (its box, then its link), so a lane that
+// takes one child reads one half.
 struct __align__(16) Node {
   float4 a;  // child0 lo.xyz, hi.x
-  float4 b;  // child0 hi.yz, child1 lo.xy
-  float4 c;  // child1 lo.z, hi.xyz
-  int4 d;    // child0, child1 (>= 0 internal node, < 0 leaf ~position), pad
+  float4 b;  // child0 hi.yz, link bits (>= 0 internal node, < 0 leaf ~position), pad
+  float4 c;  // child1 lo.xyz, hi.x
+  float4 d;  // child1 hi.yz, link bits, pad
 };
+__device__ __forceinline__ int child_link(float4 second) { return __float_as_int(second.z); }
 
 struct Ray {
   float3 o;   // rayo + tmin * rayd (shaders.slang:179, raw direction)
   float3 d;   // l2_normalize(rayd) (shaders.slang:178)
   float3 rd;  // raw rayd (SH direction)
+  float3 apex;  // rayo: the point of the ray's line that a pinhole's rays share
 };
 
 __device__ __forceinline__ Ray make_ray(float3 ro, float3 rd, float tmin) {
   Ray r;
   r.rd = rd;
+  r.apex = ro;
   r.o = make_float3(fmaf(tmin, rd.x, ro.x), fmaf(tmin, rd.y, ro.y), fmaf(tmin, rd.z, ro.z));
   const float dd = fmaf(rd.z, rd.z, fmaf(rd.y, rd.y, rd.x * rd.x));
   const float nrm = sqrtf(fmaxf(dd, kTiny));
@@ -217,9 +225,10 @@ __device__ __forceinline__ State empty_state() {
 __device__ __forceinline__ void update(State& s, float t, float4 dirac) {
   const float dt = fmaxf(t - s.t, 0.f);
   const float area = fmaxf(s.drgb.x * dt, 0.f);
-  const float rgb0 = safe_div(s.drgb.y, s.drgb.x);
-  const float rgb1 = safe_div(s.drgb.z, s.drgb.x);
-  const float rgb2 = safe_div(s.drgb.w, s.drgb.x);
+  const float inv = safe_rcp(s.drgb.x);
+  const float rgb0 = clampf(s.drgb.y * inv, kMinVal, kMaxVal);
+  const float rgb1 = clampf(s.drgb.z * inv, kMinVal, kMaxVal);
+  const float rgb2 = clampf(s.drgb.w * inv, kMinVal, kMaxVal);
   const float logT = fmaxf(area + s.logT, 0.f);
   const float w = clampf((1.f - safe_exp(-area)) * safe_exp(-s.logT), 0.f, 1.f);
   s.C.x = fmaf(w, rgb0, s.C.x);

@@ -73,6 +73,7 @@ struct FwdParams {
   EverForwardOut out;
   int frustum;  // packet kernels: frustum phase before the rounds (set from the tune)
   int stack_depth;  // traversal stack entries in use, <= kStackDepth (set from the tune)
+  int lanes;        // frustum kernels: rays per packet, <= 32 (set by the launcher)
   const float* depth_hint;  // (R) nullable: per-ray guess of the stopping t (first frustum stage)
 };
 
@@ -147,6 +148,7 @@ struct BatchFwdParams {
   int grid;            // persistent blocks
   int frustum;         // frustum phase before the rounds (set from the tune)
   int stack_depth;     // traversal stack entries in use (set from the tune)
+  int lanes;           // frustum kernel: rays per packet, a divisor of 32 (set by the launcher)
 };
 
 cudaError_t launch_forward_batched(const BatchFwdParams& P, int deg, const EverTune& tune, cudaStream_t st);

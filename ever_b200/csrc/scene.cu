@@ -410,7 +410,8 @@ __global__ void k_lbvh(const uint32_t* __restrict__ codes, int64_t N, Node* __re
     c1 = int(gamma + 1);
     parent_node[gamma + 1] = int(i);
   }
-  nodes[i].d = make_int4(c0, c1, 0, 0);
+  nodes[i].b.z = __int_as_float(c0);
+  nodes[i].d.z = __int_as_float(c1);
   if (i == 0) parent_node[0] = -1;
 }
 
@@ -420,9 +421,9 @@ __device__ __forceinline__ void child_box(const Node* nodes, const float4* aabb,
     lo = make_float3(a.x, a.y, a.z);
     hi = make_float3(b.x, b.y, b.z);
   } else {
-    const float4 a = __ldcg(&nodes[c].a), b = __ldcg(&nodes[c].b), cc = __ldcg(&nodes[c].c);
-    lo = make_float3(fminf(a.x, b.z), fminf(a.y, b.w), fminf(a.z, cc.x));
-    hi = make_float3(fmaxf(a.w, cc.y), fmaxf(b.x, cc.z), fmaxf(b.y, cc.w));
+    const float4 a = __ldcg(&nodes[c].a), b = __ldcg(&nodes[c].b), cc = __ldcg(&nodes[c].c), d = __ldcg(&nodes[c].d);
+    lo = make_float3(fminf(a.x, cc.x), fminf(a.y, cc.y), fminf(a.z, cc.z));
+    hi = make_float3(fmaxf(a.w, cc.w), fmaxf(b.x, d.x), fmaxf(b.y, d.y));
   }
 }
 
@@ -438,13 +439,14 @@ __global__ void k_refit(int64_t N, Node* __restrict__ nodes, const float4* __res
     // loads below (one instruction instead of two full fences around the atomic)
     cuda::atomic_ref<uint32_t, cuda::thread_scope_device> f(flags[n]);
     if (f.fetch_add(1u, cuda::memory_order_acq_rel) == 0u) return;  // the sibling subtree is not done yet
-    const int4 ch = __ldcg(&nodes[n].d);
+    const float c0 = __ldcg(&nodes[n].b.z), c1 = __ldcg(&nodes[n].d.z);
     float3 l0, h0, l1, h1;
-    child_box(nodes, aabb, ch.x, l0, h0);
-    child_box(nodes, aabb, ch.y, l1, h1);
+    child_box(nodes, aabb, __float_as_int(c0), l0, h0);
+    child_box(nodes, aabb, __float_as_int(c1), l1, h1);
     __stcg(&nodes[n].a, make_float4(l0.x, l0.y, l0.z, h0.x));
-    __stcg(&nodes[n].b, make_float4(h0.y, h0.z, l1.x, l1.y));
-    __stcg(&nodes[n].c, make_float4(l1.z, h1.x, h1.y, h1.z));
+    __stcg(&nodes[n].b, make_float4(h0.y, h0.z, c0, 0.f));
+    __stcg(&nodes[n].c, make_float4(l1.x, l1.y, l1.z, h1.x));
+    __stcg(&nodes[n].d, make_float4(h1.y, h1.z, c1, 0.f));
     n = parent_node[n];
   }
 }
@@ -453,9 +455,9 @@ __global__ void k_single_leaf(Node* nodes, const float4* aabb) {
   const float4 a = aabb[0], b = aabb[1];
   Node nd;
   nd.a = make_float4(a.x, a.y, a.z, b.x);
-  nd.b = make_float4(b.y, b.z, 3e38f, 3e38f);  // child 1: a far-away point box, never hit below tmax
-  nd.c = make_float4(3e38f, 3e38f, 3e38f, 3e38f);
-  nd.d = make_int4(~0, ~0, 0, 0);
+  nd.b = make_float4(b.y, b.z, __int_as_float(~0), 0.f);
+  nd.c = make_float4(3e38f, 3e38f, 3e38f, 3e38f);  // child 1: a far-away point box, never hit below tmax
+  nd.d = make_float4(3e38f, 3e38f, __int_as_float(~0), 0.f);
   nodes[0] = nd;
 }
 

@@ -582,12 +582,11 @@ __device__ void backward_ray(const BScene& S, const BRayCtx& P, int64_t r, int64
     int sp = 0, node = 0;
     for (;;) {
       const float4* np = reinterpret_cast<const float4*>(nodes + node);
-      const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-      const int4 d = __ldg(reinterpret_cast<const int4*>(np + 3));
+      const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2), d = __ldg(np + 3);
       const float3 o = ray.o;
       const bool h0 = o.x >= a.x && o.x <= a.w && o.y >= a.y && o.y <= b.x && o.z >= a.z && o.z <= b.y;
-      const bool h1 = o.x >= b.z && o.x <= c.y && o.y >= b.w && o.y <= c.z && o.z >= c.x && o.z <= c.w;
-      const int ch[2] = {d.x, d.y};
+      const bool h1 = o.x >= c.x && o.x <= c.w && o.y >= c.y && o.y <= d.x && o.z >= c.z && o.z <= d.y;
+      const int ch[2] = {child_link(b), child_link(d)};
       const bool hh[2] = {h0, h1};
       for (int k = 0; k < 2; ++k) {
         if (hh[k] && ch[k] < 0) {

@@ -44,13 +44,26 @@ __device__ __forceinline__ void buf_insert(uint64_t (&buf)[KBUF], uint64_t k) {
   }
 }
 
+// The same among the first M entries; returns the key that falls out behind them.
+template <int M, int KBUF>
+__device__ __forceinline__ uint64_t buf_insert_low(uint64_t (&buf)[KBUF], uint64_t k) {
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const uint64_t b = buf[i];
+    const bool lt = k < b;
+    buf[i] = lt ? k : b;
+    k = lt ? b : k;
+  }
+  return k;
+}
+
 __device__ __forceinline__ Node load_node(const Node* __restrict__ nodes, int n) {
   const float4* p = reinterpret_cast<const float4*>(nodes + n);
   Node nd;
   nd.a = __ldg(p + 0);
   nd.b = __ldg(p + 1);
   nd.c = __ldg(p + 2);
-  nd.d = __ldg(reinterpret_cast<const int4*>(p + 3));
+  nd.d = __ldg(p + 3);
   return nd;
 }
 
@@ -112,8 +125,8 @@ __device__ void gather_ray(const Node* __restrict__ nodes, const Record* __restr
     const Node nd = load_node(nodes, node);
     const float hi = fminf(cap, key_t(buf[KBUF - 1]));  // an empty slot is NaN: fminf keeps cap
     const float tc[2] = {slab(sl, nd.a.x, nd.a.y, nd.a.z, nd.a.w, nd.b.x, nd.b.y, lo_t, hi),
-                         slab(sl, nd.b.z, nd.b.w, nd.c.x, nd.c.y, nd.c.z, nd.c.w, lo_t, hi)};
-    const int c[2] = {nd.d.x, nd.d.y};
+                         slab(sl, nd.c.x, nd.c.y, nd.c.z, nd.c.w, nd.d.x, nd.d.y, lo_t, hi)};
+    const int c[2] = {child_link(nd.b), child_link(nd.d)};
 #pragma unroll
     for (int k = 0; k < 2; ++k)
       if (tc[k] != INFINITY && c[k] < 0) leaf_insert(recs, ~c[k], ray, lower, s16, tmax, buf);
@@ -163,11 +176,11 @@ __device__ void gather_packet(const Node* __restrict__ nodes, const Record* __re
     if (act) {
       const float hi = fminf(cap, key_t(buf[KBUF - 1]));
       t0 = slab(sl, nd.a.x, nd.a.y, nd.a.z, nd.a.w, nd.b.x, nd.b.y, lo_t, hi);
-      t1 = slab(sl, nd.b.z, nd.b.w, nd.c.x, nd.c.y, nd.c.z, nd.c.w, lo_t, hi);
+      t1 = slab(sl, nd.c.x, nd.c.y, nd.c.z, nd.c.w, nd.d.x, nd.d.y, lo_t, hi);
     }
     const unsigned m0 = __ballot_sync(kFull, t0 != INFINITY);
     const unsigned m1 = __ballot_sync(kFull, t1 != INFINITY);
-    const int c0 = nd.d.x, c1 = nd.d.y;
+    const int c0 = child_link(nd.b), c1 = child_link(nd.d);
     if (c0 < 0 && t0 != INFINITY) leaf_insert(recs, ~c0, ray, lower, s16, tmax, buf);
     if (c1 < 0 && t1 != INFINITY) leaf_insert(recs, ~c1, ray, lower, s16, tmax, buf);
     const bool g0 = c0 >= 0 && m0 != 0u, g1 = c1 >= 0 && m1 != 0u;
@@ -250,8 +263,8 @@ __device__ int point_members(const Node* __restrict__ nodes, const Record* __res
   for (;;) {
     const Node nd = load_node(nodes, node);
     const bool h0 = act && box_contains(nd.a.x, nd.a.y, nd.a.z, nd.a.w, nd.b.x, nd.b.y, ray.o);
-    const bool h1 = act && box_contains(nd.b.z, nd.b.w, nd.c.x, nd.c.y, nd.c.z, nd.c.w, ray.o);
-    const int c0 = nd.d.x, c1 = nd.d.y;
+    const bool h1 = act && box_contains(nd.c.x, nd.c.y, nd.c.z, nd.c.w, nd.d.x, nd.d.y, ray.o);
+    const int c0 = child_link(nd.b), c1 = child_link(nd.d);
     if (h0 && c0 < 0) point_leaf<DEG>(recs, order, feats, fst, B, bs, ray, ~c0, n_mem, mem_p, mem_j, extra, status);
     if (h1 && c1 < 0) point_leaf<DEG>(recs, order, feats, fst, B, bs, ray, ~c1, n_mem, mem_p, mem_j, extra, status);
     bool g0 = h0 && c0 >= 0, g1 = h1 && c1 >= 0;
@@ -293,7 +306,6 @@ struct TraceCtx {
   float tmin, tmax;
   int max_iters;
   EverForwardOut out;
-  bool frustum;        // packet kernels: run the frustum phase before the rounds
   int depth;           // traversal stack entries in use (<= kStackDepth)
   const float* depth_hint;  // (R) nullable: per-ray guess of the stopping t
 };
@@ -425,7 +437,7 @@ __global__ void __launch_bounds__(256) k_trace_fwd_ray(const FwdParams P) {
   if (gi >= P.R) return;
   const int64_t r = P.ray_order ? int64_t(P.ray_order[gi]) : gi;
   const SceneRef sc = scene_of(P);
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.frustum != 0, P.stack_depth, P.depth_hint};
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
   const Ray ray = load_ray(P.rayo, P.rayd, r, P.tmin);
   const RaySlab sl = make_slab(ray);
   float B[16];
@@ -522,176 +534,388 @@ __device__ __forceinline__ bool run_rounds(const SceneRef& sc, const TraceCtx& C
 }
 
 // ---- packet frustum phase ----
-// The warp bounds its active rays by intervals (origins, directions, inverse directions),
-// walks the BVH breadth first with one node per lane, keeping every child box some packet
-// ray can meet (a conservative interval slab test), and lists the leaves sorted by the
-// earliest t at which any packet ray can enter them. Every lane then takes the leaves in
-// that order: the leaf's events on its own ray go into its sorted buffer, and before the
-// next leaf, whose events all lie at or beyond that leaf's entry bound T, the events
-// below T are final and are integrated in order. So each ray integrates exactly its
-// sorted event sequence, as the rounds do, with one walk per packet instead of one per
-// round, and the box tests spread over the lanes instead of repeating for every ray.
-// A lane whose buffer would overflow, and every lane of a packet whose breadth-first
-// lists overflow shared memory, stops after its last integrated event; the rounds then
-// continue it from there (lower = that event's key), so the results do not depend on it.
-// Events a lane holds in the frustum phase. Fewer than the rounds' buffer: the phase's
-// buffer lives across the whole leaf loop, and 12 of 16 gave the shortest forward at 1M
-// ellipsoids / 1080p (5.90 ms; 16: 6.22, 8: 6.85, 24: 7.13 ms with spills).
-constexpr int frustum_buffer(int kbuf) { return kbuf == 16 ? 12 : kbuf; }
-constexpr int kFrontierCap = 384;  // nodes per breadth-first level
-constexpr int kCandCap = 512;      // leaves per packet (a power of two: the sort's width)
-// Shared ints per warp: the traversal stack, two frontier levels, the leaf keys (64-bit).
-constexpr int kWarpInts = kStackDepth + 2 * kFrontierCap + 2 * kCandCap;
+// Bound by issued instructions (55% of the issue slots busy, ALU pipe 42%, DRAM 1%), so the
+// phase is cut into steps that each keep the lanes busy:
+//  - list_leaves: the warp bounds its rays by intervals (origins, inverse directions), walks
+//    the BVH with one child box per lane and lists the leaves whose box some ray can meet;
+//    each lane then tests one listed ellipsoid against the cone of the packet's
+//    directions, which drops 40% of them (boxes of thin turned ellipsoids are mostly
+//    empty), and the rest are sorted by the earliest t at which any ray can enter them;
+//  - every lane tests the leaves in that order; a leaf's events on the lane's ray go into
+//    its sorted buffer, and before the next leaf, whose events all lie at or beyond that
+//    leaf's entry bound T, the events below T are final;
+//  - order_events takes the final events in order, decides where the ray ends and logs them;
+//  - ring_integrate integrates them later, most lanes at once.
+// So each ray integrates exactly its sorted event sequence, as the rounds do. Where the
+// leaves of the whole t range do not fit, the phase goes on in stages over t. At 1M
+// ellipsoids / 1080p the forward's kernels took 6.26 ms before (one walk over whole nodes,
+// no cone test, integration where an event became final, a second pass of stack rounds for
+// overflowing packets) and take 3.6 ms; a packet issues 34k instructions, 66k before.
+// Rays in no order (no_order) have no list in common and go to the rounds at once.
+// Events a lane holds in the frustum phase. More only cost registers: at 1M ellipsoids /
+// 1080p a lane holds more than 5 on 3% of the leaves, and a lane that runs out makes another
+// pass over the list (8: 3.6 ms, 12: 4.1 ms).
+constexpr int frustum_buffer(int kbuf) { return kbuf == 32 ? 16 : 8; }
+constexpr int kLowEvents = 2;      // buffered events up to which an insertion moves only the first entries
+constexpr int kHold = 4;           // leaves between two rounds of ordering
+constexpr int kWalkCap = 256;      // nodes waiting in the walk
+constexpr int kFirstLeaves = 128;  // leaves of a group's first stage
+constexpr int kStageLeaves = 256;  // leaves of a later stage
+constexpr int kCandCap = kStageLeaves + 64;
+constexpr int kMaxCuts = 6;      // of a list that overflows in one walk
+constexpr int kMaxStages = 128;  // then the rounds take over
+constexpr int kTileWords = 24;
+constexpr int kStateWords = 14;  // of a lane's integration state: State (13), the last event's id
+// Shared ints per warp: the walk's nodes with their entry bounds (before and after it, the
+// traversal stack of the rounds; after it, the events' ring),
+// the leaf keys (64-bit), the lanes' integration state, the packet's direction tile.
+constexpr int kWarpInts = 2 * kWalkCap + 2 * kCandCap + kStateWords * 32 + kTileWords;
 
-__device__ __forceinline__ uint32_t ordered_bits(float f) {
-  const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+// Warp minimum / maximum; NaN lanes are ignored (a NaN ray meets nothing).
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
-__device__ __forceinline__ float from_ordered(uint32_t u) {
-  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
-__device__ __forceinline__ float warp_min(float v) { return from_ordered(__reduce_min_sync(kFull, ordered_bits(v))); }
-__device__ __forceinline__ float warp_max(float v) { return from_ordered(__reduce_max_sync(kFull, ordered_bits(v))); }
+__device__ __forceinline__ float rcp_approx(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
 
+// Interval bounds of a packet's rays for the box test. On an axis whose directions share a
+// sign, every ray enters a box through one plane (the upper one where the sign is negative)
+// and leaves it through the other, and the bound of the entry comes from one end of the
+// origins' interval: o_near; that of the exit from the other: o_far.
 struct PacketBounds {
-  float omin[3], omax[3];  // origins
+  float o_near[3], o_far[3];
   float imin[3], imax[3];  // inverse directions (as the per-ray slab test takes them)
-  float dmin[3], dmax[3];  // unit directions
-  unsigned free_axes;      // axes whose direction changes sign within the packet
+  unsigned neg, free;      // axes with negative directions / with directions of both signs
 };
 
-// Interval bounds over the lanes with `part` (all lanes take part in the reductions).
-__device__ __forceinline__ PacketBounds packet_bounds(const Ray& ray, const RaySlab& sl, bool part) {
+// The packet's rays as a cone of directions, and the origin and direction intervals that
+// the free axes need; one copy per warp in shared memory.
+struct PacketTile {
+  float o[3];      // the common point of the rays' lines (their origin before the tmin shift)
+  float d0[3];     // centre direction; every ray's direction is a multiple of
+  float e1[3];     //   d0 + a e1 + b e2 with |a|, |b| <= 1
+  float e2[3];
+  float omin[3], omax[3], dmin[3], dmax[3];  // free axes only
+};
+static_assert(sizeof(PacketTile) <= kTileWords * sizeof(int), "tile words");
+
+// Bounds over the lanes with `part` (all lanes take part in the reductions). Writes the tile;
+// *area: its size, +inf when there is none (no common apex, or no narrow cone).
+__device__ __forceinline__ PacketBounds packet_bounds(const Ray& ray, const RaySlab& sl, bool part, PacketTile* tile,
+                                                      int lane, float* area) {
   PacketBounds P;
   const float o[3] = {ray.o.x, ray.o.y, ray.o.z}, d[3] = {ray.d.x, ray.d.y, ray.d.z};
-  const float iv[3] = {sl.invd.x, sl.invd.y, sl.invd.z};
-  P.free_axes = 0;
+  const float iv[3] = {sl.invd.x, sl.invd.y, sl.invd.z}, ap[3] = {ray.apex.x, ray.apex.y, ray.apex.z};
+  P.neg = P.free = 0;
+  bool common = true;
+  float m[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    P.omin[a] = warp_min(part ? o[a] : INFINITY);
-    P.omax[a] = warp_max(part ? o[a] : -INFINITY);
+    const float omin = warp_min(part ? o[a] : INFINITY), omax = warp_max(part ? o[a] : -INFINITY);
+    const float dmin = warp_min(part ? d[a] : INFINITY), dmax = warp_max(part ? d[a] : -INFINITY);
+    const float amin = warp_min(part ? ap[a] : INFINITY), amax = warp_max(part ? ap[a] : -INFINITY);
     P.imin[a] = warp_min(part ? iv[a] : INFINITY);
     P.imax[a] = warp_max(part ? iv[a] : -INFINITY);
-    P.dmin[a] = warp_min(part ? d[a] : INFINITY);
-    P.dmax[a] = warp_max(part ? d[a] : -INFINITY);
-    if (P.imin[a] < 0.f && P.imax[a] > 0.f) P.free_axes |= 1u << a;
+    const bool neg = P.imax[a] < 0.f;
+    if (neg) P.neg |= 1u << a;
+    if (P.imin[a] < 0.f && P.imax[a] > 0.f) P.free |= 1u << a;
+    P.o_near[a] = neg ? omin : omax;
+    P.o_far[a] = neg ? omax : omin;
+    common = common && amin == amax;
+    m[a] = 0.5f * (dmin + dmax);
+    if (lane == 0) {
+      tile->o[a] = amin;
+      tile->omin[a] = omin;
+      tile->omax[a] = omax;
+      tile->dmin[a] = dmin;
+      tile->dmax[a] = dmax;
+    }
   }
+  // tangent plane of the middle direction, and the rays' rectangle in it: the smallest over a
+  // few rotations. Only a bound is needed, so approximate reciprocals do (margins below).
+  const float inv_m = rsqrtf(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) m[a] *= inv_m;
+  const bool x_small = fabsf(m[0]) < 0.6f;
+  float t1[3], t2[3];
+  {  // t1 = m x axis
+    const float ax = x_small ? 1.f : 0.f, ay = x_small ? 0.f : 1.f;
+    t1[0] = -m[2] * ay;
+    t1[1] = m[2] * ax;
+    t1[2] = m[0] * ay - m[1] * ax;
+    const float n = rsqrtf(t1[0] * t1[0] + t1[1] * t1[1] + t1[2] * t1[2]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) t1[a] *= n;
+    t2[0] = m[1] * t1[2] - m[2] * t1[1];
+    t2[1] = m[2] * t1[0] - m[0] * t1[2];
+    t2[2] = m[0] * t1[1] - m[1] * t1[0];
+  }
+  const float dm = d[0] * m[0] + d[1] * m[1] + d[2] * m[2];
+  const float k = 1.f / dm;
+  const float u = (d[0] * t1[0] + d[1] * t1[1] + d[2] * t1[2]) * k;
+  const float v = (d[0] * t2[0] + d[1] * t2[1] + d[2] * t2[2]) * k;
+  float best = INFINITY, uc = 0.f, vc = 0.f, uh = 0.f, vh = 0.f, bc = 1.f, bs = 0.f;
+  float cq = 1.f, sq = 0.f;
+#pragma unroll 1
+  for (int q = 0; q < 4; ++q) {  // 0, 22.5, 45, 67.5 degrees
+    const float x = cq * u + sq * v, y = cq * v - sq * u;
+    const float x0 = warp_min(part ? x : INFINITY), x1 = warp_max(part ? x : -INFINITY);
+    const float y0 = warp_min(part ? y : INFINITY), y1 = warp_max(part ? y : -INFINITY);
+    const float a = (x1 - x0) * (y1 - y0);
+    if (a < best) {
+      best = a;
+      uc = 0.5f * (x0 + x1);
+      vc = 0.5f * (y0 + y1);
+      uh = 0.5f * (x1 - x0);
+      vh = 0.5f * (y1 - y0);
+      bc = cq;
+      bs = sq;
+    }
+    const float c = cq * 0.92387953f - sq * 0.38268343f;
+    sq = cq * 0.38268343f + sq * 0.92387953f;
+    cq = c;
+  }
+  // directions carry a few float roundings: 1e-6 of the unit tangent plane covers them
+  uh = uh * 1.00001f + 1e-6f;
+  vh = vh * 1.00001f + 1e-6f;
+  *area = common && warp_min(part ? dm : INFINITY) > 0.5f ? uh * vh : INFINITY;
+  if (lane == 0) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float r1 = bc * t1[a] + bs * t2[a], r2 = bc * t2[a] - bs * t1[a];
+      tile->d0[a] = m[a] + uc * r1 + vc * r2;
+      tile->e1[a] = uh * r1;
+      tile->e2[a] = vh * r2;
+    }
+  }
+  __syncwarp();
   return P;
 }
 
-__device__ __forceinline__ float min4(float a, float b, float c, float d) { return fminf(fminf(a, b), fminf(c, d)); }
-__device__ __forceinline__ float max4(float a, float b, float c, float d) { return fmaxf(fmaxf(a, b), fmaxf(c, d)); }
-
-// A lower bound of the t at which any packet ray enters the box within [0, cap], or +inf
+// A lower bound of the t at which any packet ray is in the box within [t_lo, cap], or +inf
 // when no packet ray can meet it there. Interval products bound every ray's plane
 // distances; the float rounding of the bound (a few ulps) is covered by widening it by a
 // relative 1e-6. Axes whose direction changes sign bound no t: there the positions the
 // packet reaches over the t range of the other axes must overlap the box.
-__device__ __forceinline__ float packet_entry(const PacketBounds& P, float lx, float ly, float lz, float hx, float hy,
-                                              float hz, float cap) {
-  const float lo[3] = {lx, ly, lz}, hi[3] = {hx, hy, hz};
+__device__ __forceinline__ float packet_entry(const PacketBounds& P, const PacketTile* tile, float4 a, float4 b,
+                                              float t_lo, float cap) {
+  const float lo[3] = {a.x, a.y, a.z}, hi[3] = {a.w, b.x, b.y};
   float tn = 0.f, tf = cap;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    if (P.free_axes >> a & 1u) continue;
-    const float d0 = lo[a] - P.omax[a], d1 = lo[a] - P.omin[a];
-    const float e0 = hi[a] - P.omax[a], e1 = hi[a] - P.omin[a];
-    const float p0 = d0 * P.imin[a], p1 = d0 * P.imax[a], p2 = d1 * P.imin[a], p3 = d1 * P.imax[a];
-    const float q0 = e0 * P.imin[a], q1 = e0 * P.imax[a], q2 = e1 * P.imin[a], q3 = e1 * P.imax[a];
-    tn = fmaxf(tn, fminf(min4(p0, p1, p2, p3), min4(q0, q1, q2, q3)));
-    tf = fminf(tf, fmaxf(max4(p0, p1, p2, p3), max4(q0, q1, q2, q3)));
-  }
-  tn = tn - 1e-6f * fabsf(tn);
-  tf = tf + 1e-6f * fabsf(tf);
-  if (!(tn <= tf)) return INFINITY;
-  if (P.free_axes) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      if (!(P.free_axes >> a & 1u)) continue;
-      const float xl = P.omin[a] + min4(tn * P.dmin[a], tn * P.dmax[a], tf * P.dmin[a], tf * P.dmax[a]);
-      const float xh = P.omax[a] + max4(tn * P.dmin[a], tn * P.dmax[a], tf * P.dmin[a], tf * P.dmax[a]);
-      const float tol = 1e-6f * (fabsf(xl) + fabsf(xh) + fabsf(tf));
-      if (xh + tol < lo[a] || xl - tol > hi[a]) return INFINITY;
+  for (int q = 0; q < 3; ++q) {
+    const bool neg = P.neg >> q & 1u;
+    const float dn = (neg ? hi[q] : lo[q]) - P.o_near[q], df = (neg ? lo[q] : hi[q]) - P.o_far[q];
+    const float n = fminf(dn * P.imin[q], dn * P.imax[q]), f = fmaxf(df * P.imin[q], df * P.imax[q]);
+    if (!(P.free >> q & 1u)) {
+      tn = fmaxf(tn, n);
+      tf = fminf(tf, f);
     }
   }
-  return fmaxf(tn, 0.f);
+  tn = fmaxf(tn * 0.999999f, t_lo);  // tn >= 0; a product, so that an infinite bound stays one
+  tf = tf + 1e-6f * fabsf(tf);
+  if (!(tn <= tf)) return INFINITY;
+  if (P.free) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      if (!(P.free >> q & 1u)) continue;
+      const float d0 = tile->dmin[q], d1 = tile->dmax[q];
+      const float xl = tile->omin[q] + fminf(fminf(tn * d0, tn * d1), fminf(tf * d0, tf * d1));
+      const float xh = tile->omax[q] + fmaxf(fmaxf(tn * d0, tn * d1), fmaxf(tf * d0, tf * d1));
+      const float tol = 1e-6f * (fabsf(xl) + fabsf(xh) + fabsf(tf));
+      if (xh + tol < lo[q] || xl - tol > hi[q]) return INFINITY;
+    }
+  }
+  return tn;
 }
 
-// Breadth-first walk: the leaf keys (entry bound bits << 32 | position) of every leaf the
-// packet can meet, into cand[0, n). Returns n, or -1 when a level or the leaf list does
-// not fit its shared-memory capacity.
-__device__ __forceinline__ int packet_leaves(const Node* __restrict__ nodes, const PacketBounds& P, float cap,
-                                             int* front, uint64_t* cand, int lane) {
-  int* cur = front;
-  int* nxt = front + kFrontierCap;
-  if (lane == 0) cur[0] = 0;
-  __syncwarp();
-  int nf = 1, nc = 0;
-  const unsigned below = (1u << lane) - 1u;
-  for (int level = 0; nf > 0; ++level) {
-    if (level >= 4 * kStackDepth) return -1;  // deeper than any tree the build makes
-    int nn = 0;
-    for (int base = 0; base < nf; base += 32) {
-      const int i = base + lane;
-      float te0 = INFINITY, te1 = INFINITY;
-      int c0 = 0, c1 = 0;
-      if (i < nf) {
-        const Node nd = load_node(nodes, cur[i]);
-        te0 = packet_entry(P, nd.a.x, nd.a.y, nd.a.z, nd.a.w, nd.b.x, nd.b.y, cap);
-        te1 = packet_entry(P, nd.b.z, nd.b.w, nd.c.x, nd.c.y, nd.c.z, nd.c.w, cap);
-        c0 = nd.d.x;
-        c1 = nd.d.y;
-      }
+// Whether no ray of the packet's tile can meet ellipsoid j. In the ellipsoid's frame (unit
+// sphere) the rays start at c and run along v0 + a v1 + b v2, |a|, |b| <= 1. They cross the
+// plane through the centre normal to v0 in l + s' (a v1' + b v2'), v1' and v2' the parts of
+// v1, v2 normal to v0, s' = s / (1 + a p1 + b p2): a parallelogram, once s' is replaced by
+// its largest value. A ray's distance from the centre is at least its crossing point's
+// times the cosine of its angle to v0, so the packet misses when the parallelogram stays
+// farther than 1 / cos from the centre. The margins cover the float rounding here and in
+// the exact test (both about 1e-6 |c| of the radius); NaN never rejects.
+__device__ __forceinline__ bool packet_misses(const PacketTile* T, const Record* __restrict__ recs, int j) {
+  const float4* rp = reinterpret_cast<const float4*>(recs + j);
+  const float4 r[3] = {__ldg(rp), __ldg(rp + 1), __ldg(rp + 2)};
+  const float x = T->o[0] - r[0].w, y = T->o[1] - r[1].w, z = T->o[2] - r[2].w;
+  float c[3], v0[3], v1[3], v2[3];
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const float te = k ? te1 : te0;
-        const int c = k ? c1 : c0;
-        const bool hit = te != INFINITY;
-        const unsigned mi = __ballot_sync(kFull, hit && c >= 0);
-        const unsigned ml = __ballot_sync(kFull, hit && c < 0);
-        if (hit && c >= 0) {
-          const int q = nn + __popc(mi & below);
-          if (q < kFrontierCap) nxt[q] = c;
-        }
-        if (hit && c < 0) {
-          const int q = nc + __popc(ml & below);
-          if (q < kCandCap) cand[q] = (uint64_t(__float_as_uint(te)) << 32) | uint32_t(~c);
-        }
-        nn += __popc(mi);
-        nc += __popc(ml);
+  for (int i = 0; i < 3; ++i) {
+    c[i] = fmaf(r[i].z, z, fmaf(r[i].y, y, r[i].x * x));
+    v0[i] = fmaf(r[i].z, T->d0[2], fmaf(r[i].y, T->d0[1], r[i].x * T->d0[0]));
+    v1[i] = fmaf(r[i].z, T->e1[2], fmaf(r[i].y, T->e1[1], r[i].x * T->e1[0]));
+    v2[i] = fmaf(r[i].z, T->e2[2], fmaf(r[i].y, T->e2[1], r[i].x * T->e2[0]));
+  }
+  auto dot = [](const float (&p)[3], const float (&q)[3]) { return fmaf(p[2], q[2], fmaf(p[1], q[1], p[0] * q[0])); };
+  const float iv = rcp_approx(dot(v0, v0));
+  const float s = -dot(c, v0) * iv, p1 = dot(v1, v0) * iv, p2 = dot(v2, v0) * iv;
+  const float g = fabsf(p1) + fabsf(p2);
+  float l[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    l[i] = fmaf(s, v0[i], c[i]);
+    v1[i] = fmaf(-p1, v0[i], v1[i]);
+    v2[i] = fmaf(-p2, v0[i], v2[i]);
+  }
+  const float k = rcp_approx(1.f - g), sk = s * k;
+  const float q11 = dot(v1, v1), q22 = dot(v2, v2);
+  const float tan2 = 2.f * (q11 + q22) * iv * k * k;
+  const float A = dot(l, l), B1 = sk * dot(l, v1), B2 = sk * dot(l, v2), s2 = sk * sk;
+  const float C11 = s2 * q11, C22 = s2 * q22, C12 = s2 * dot(v1, v2);
+  const float det = C11 * C22 - C12 * C12;
+  const bool inside = fabsf(B2 * C12 - B1 * C22) <= det && fabsf(B1 * C12 - B2 * C11) <= det;
+  const float i1 = rcp_approx(C11), i2 = rcp_approx(C22);
+  float f = INFINITY;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const float sg = e ? -1.f : 1.f;
+    const float h1 = fmaf(sg, C12, B1), h2 = fmaf(sg, C12, B2);
+    const float a = clampf(-h1 * i1, -1.f, 1.f), b = clampf(-h2 * i2, -1.f, 1.f);
+    f = fminf(f, fmaf(a, fmaf(a, C11, 2.f * h1), fmaf(2.f * sg, B2, A + C22)));
+    f = fminf(f, fmaf(b, fmaf(b, C22, 2.f * h2), fmaf(2.f * sg, B1, A + C11)));
+  }
+  const float size = fabsf(c[0]) + fabsf(c[1]) + fabsf(c[2]);
+  const float lim = (1.f + tan2) * (1.002f + 1e-5f * size) + 4e-6f * (A + C11 + C22);
+  return g < 0.5f && !inside && f > lim && C11 + C22 < 1e5f;
+}
+
+// Drops the leaves that the packet's tile misses from cand[0, n), keeping the others.
+__device__ __forceinline__ int cull_leaves(const PacketTile* tile, const Record* __restrict__ recs, uint64_t* cand,
+                                           int from, int n, int lane) {
+  int kept = from;
+  const unsigned below = (1u << lane) - 1u;
+#pragma unroll 1
+  for (int base = from; base < n; base += 32) {
+    const int i = base + lane;
+    uint64_t key = kEmptyKey;
+    bool keep = false;
+    if (i < n) {
+      key = cand[i];
+      keep = !packet_misses(tile, recs, int(uint32_t(key)));
+    }
+    const unsigned m = __ballot_sync(kFull, keep);
+    __syncwarp();
+    if (keep) cand[kept + __popc(m & below)] = key;
+    kept += __popc(m);
+  }
+  __syncwarp();
+  return kept;
+}
+
+// Keeps the nearest `least` to `most` (ties permitting) of cand[0, n) and returns their
+// number; every dropped leaf's entry bound is at least *cut. 0 when all entry bounds are equal.
+__device__ __forceinline__ int nearer_leaves(uint64_t* cand, int n, int least, int most, int lane, float* cut) {
+  uint32_t lo = 0, hi = 0x7f800000u;  // fewer than `least` bounds lie below lo, more than `most` below hi
+  int kept = 0;
+  uint32_t at = 0;
+  while (hi - lo > 1) {
+    at = lo + (hi - lo) / 2;
+    int c = 0;
+    for (int i = lane; i < n; i += 32) c += uint32_t(cand[i] >> 32) < at ? 1 : 0;
+    kept = __reduce_add_sync(kFull, c);
+    if (kept < least) lo = at;
+    else if (kept > most) hi = at;
+    else break;
+  }
+  if (kept < least || kept > most) {  // a run of equal bounds spans the range: cut below or above it
+    int below = 0;
+    for (int i = lane; i < n; i += 32) below += uint32_t(cand[i] >> 32) < lo ? 1 : 0;
+    at = __reduce_add_sync(kFull, below) > 0 ? lo : hi;
+  }
+  *cut = __uint_as_float(at);
+  int out = 0;
+  const unsigned under = (1u << lane) - 1u;
+  for (int base = 0; base < n; base += 32) {
+    const int i = base + lane;
+    const uint64_t key = i < n ? cand[i] : kEmptyKey;
+    const bool keep = uint32_t(key >> 32) < at;
+    const unsigned m = __ballot_sync(kFull, keep);
+    __syncwarp();
+    if (keep) cand[out + __popc(m & under)] = key;
+    out += __popc(m);
+  }
+  __syncwarp();
+  return out < n ? out : 0;
+}
+
+// Walk of the BVH with one child box per lane and 32 nodes at a time (two boxes per lane
+// in flight: the walk waits on its loads), nearer siblings first, from a stack of nodes and
+// their entry bounds in shared memory. Lists the leaf keys (entry bound bits << 32 |
+// position) of the leaves the packet can meet within [t_lo, *cap] in cand[0, n). When more
+// than `limit` remain, the nearest are kept and *cap is lowered to where they end. Returns
+// n <= limit, or -1 when no cut clearly beyond t_lo leaves few enough (many leaves reach
+// back to t_lo: stages would hardly advance) or too many cuts were needed (a group this
+// wide gains nothing from a common list).
+__device__ __forceinline__ int packet_leaves(const Node* __restrict__ nodes, const Record* __restrict__ recs,
+                                             const PacketBounds& P, const PacketTile* tile, bool cull, float t_lo,
+                                             float* cap, int limit, int* stack, uint64_t* cand, int lane) {
+  float* bound = reinterpret_cast<float*>(stack + kWalkCap);
+  if (lane == 0) {
+    stack[0] = 0;
+    bound[0] = t_lo;
+  }
+  __syncwarp();
+  int sp = 1, nc = 0, checked = 0, cuts = 0;
+  const unsigned below = (1u << lane) - 1u;
+#pragma unroll 1
+  while (sp > 0) {
+    const int take = min(min(sp, 32), kWalkCap - sp);
+    if (take == 0) return -1;
+    sp -= take;
+    float4 a[2], b[2];
+    bool on[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = 16 * k + (lane >> 1);
+      on[k] = i < take && bound[sp + i] <= *cap;
+      if (on[k]) {
+        const float4* p = reinterpret_cast<const float4*>(nodes + stack[sp + i]) + 2 * (lane & 1);
+        a[k] = __ldg(p);
+        b[k] = __ldg(p + 1);
       }
     }
     __syncwarp();
-    if (nn > kFrontierCap || nc > kCandCap) return -1;
-    int* t = cur;
-    cur = nxt;
-    nxt = t;
-    nf = nn;
-  }
-  return nc;
-}
-
-// Ascending bitonic sort of cand[0, n) in shared memory by the warp (n <= kCandCap).
-__device__ __forceinline__ void sort_keys_smem(uint64_t* cand, int n, int lane) {
-  int w = 32;
-  while (w < n) w <<= 1;
-  for (int i = n + lane; i < w; i += 32) cand[i] = kEmptyKey;
-  __syncwarp();
-  for (int k = 2; k <= w; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < w; i += 32) {
-        const int l = i ^ j;
-        if (l > i) {
-          const uint64_t a = cand[i], b = cand[l];
-          if ((a > b) == ((i & k) == 0)) {
-            cand[i] = b;
-            cand[l] = a;
-          }
-        }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (k == 1 && take <= 16) break;
+      const float te = on[k] ? packet_entry(P, tile, a[k], b[k], t_lo, *cap) : INFINITY;
+      const int c = on[k] ? child_link(b[k]) : 0;
+      const bool hit = te != INFINITY, in = hit && c >= 0, leaf = hit && c < 0;
+      const float sib = __shfl_xor_sync(kFull, te, 1);
+      const bool near = te < sib || (te == sib && (lane & 1));
+      const unsigned mf = __ballot_sync(kFull, in && !near), mn = __ballot_sync(kFull, in && near);
+      const unsigned ml = __ballot_sync(kFull, leaf);
+      if (in) {
+        const int q = sp + (near ? __popc(mf) + __popc(mn & below) : __popc(mf & below));
+        stack[q] = c;
+        bound[q] = te;
       }
-      __syncwarp();
+      if (leaf) cand[nc + __popc(ml & below)] = (uint64_t(__float_as_uint(te)) << 32) | uint32_t(~c);
+      sp += __popc(mf) + __popc(mn);
+      nc += __popc(ml);
+    }
+    __syncwarp();
+    if (nc > limit || sp == 0) {
+      if (cull) nc = checked = cull_leaves(tile, recs, cand, checked, nc, lane);
+      if (nc > limit) {
+        nc = checked = nearer_leaves(cand, nc, limit / 2, limit - limit / 8, lane, cap);
+        if (nc == 0 || nc > limit || !(*cap > 1.001f * t_lo + 1e-6f) || ++cuts > kMaxCuts) return -1;
+      }
     }
   }
+  return nc;
 }
 
 __device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, int m) {
@@ -699,146 +923,451 @@ __device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, int m) {
   return (uint64_t(hi) << 32) | lo;
 }
 
-// Ascending bitonic sort of 32 * E keys held E per lane (key lane * E + r in k[r]): the
-// stages whose partners lie in the same lane compare-swap registers, the others exchange
-// with lane ^ (stride / E) by shuffles. No shared memory, no warp barriers.
-template <int E>
-__device__ __forceinline__ void sort_regs(uint64_t (&k)[E], int lane) {
-#pragma unroll
-  for (int size = 2; size <= 32 * E; size <<= 1) {
-#pragma unroll
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      if (stride < E) {
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-          const int q = r ^ stride;
-          if (q > r) {
-            const bool up = ((lane * E + r) & size) == 0;
-            const uint64_t a = k[r], b = k[q];
-            const bool sw = (a > b) == up;
-            k[r] = sw ? b : a;
-            k[q] = sw ? a : b;
-          }
-        }
-      } else {
-        const int m = stride / E;
-        const bool lower = (lane & m) == 0;
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-          const uint64_t o = shfl_xor64(k[r], m);
-          const bool up = ((lane * E + r) & size) == 0;
-          const bool take_min = lower == up;
-          k[r] = take_min ? (o < k[r] ? o : k[r]) : (o > k[r] ? o : k[r]);
-        }
-      }
-    }
-  }
-}
-
-// Sorts cand[0, n) ascending (n <= 32 * E) through registers.
+// Sorts cand[0, n) ascending (n <= 32 * E): bitonic, key r * 32 + lane in register r, strides
+// below 32 by shuffles, the others inside the lane. The stage loops stay rolled: unrolled
+// they are thousands of instructions that run once per packet, and the instruction cache
+// misses cost more than the loops.
 template <int E>
 __device__ __forceinline__ void sort_keys_r(uint64_t* cand, int n, int lane) {
   uint64_t k[E];
 #pragma unroll
-  for (int r = 0; r < E; ++r) {
-    const int i = lane * E + r;
-    k[r] = i < n ? cand[i] : kEmptyKey;
+  for (int r = 0; r < E; ++r) k[r] = 32 * r + lane < n ? cand[32 * r + lane] : kEmptyKey;
+#pragma unroll 1
+  for (int size = 2; size <= 32 * E; size <<= 1) {
+#pragma unroll
+    for (int d = E / 2; d > 0; d >>= 1) {  // stride 32 d
+      if (size <= 32 * d) continue;
+#pragma unroll
+      for (int r = 0; r < E; ++r) {
+        if (r & d) continue;
+        const bool up = ((32 * r) & size) == 0;
+        const uint64_t x = k[r], y = k[r | d];
+        const bool sw = (x > y) == up;
+        k[r] = sw ? y : x;
+        k[r | d] = sw ? x : y;
+      }
+    }
+#pragma unroll 1
+    for (int stride = min(size >> 1, 16); stride > 0; stride >>= 1) {
+      const bool lower = (lane & stride) == 0;
+#pragma unroll
+      for (int r = 0; r < E; ++r) {
+        const uint64_t o = shfl_xor64(k[r], stride);
+        const bool up = ((32 * r + lane) & size) == 0;
+        const bool less = o < k[r];
+        k[r] = (less == (lower == up)) ? o : k[r];
+      }
+    }
   }
-  sort_regs<E>(k, lane);
   __syncwarp();
 #pragma unroll
-  for (int r = 0; r < E; ++r) cand[lane * E + r] = k[r];
+  for (int r = 0; r < E; ++r) cand[32 * r + lane] = k[r];
   __syncwarp();
 }
-// Up to 256 keys sort in registers; longer lists in shared memory.
 __device__ __forceinline__ void sort_keys(uint64_t* cand, int n, int lane) {
-  if (n <= 32 * 4) sort_keys_r<4>(cand, n, lane);
-  else if (n <= 32 * 8) sort_keys_r<8>(cand, n, lane);
-  else sort_keys_smem(cand, n, lane);
+  if (n <= 64) sort_keys_r<2>(cand, n, lane);
+  else if (n <= 128) sort_keys_r<4>(cand, n, lane);
+  else sort_keys_r<8>(cand, n, lane);
+}
+static_assert(kStageLeaves <= 256, "sort_keys takes up to 256 keys");
+
+// The sorted leaf list of a group of the warp's rays (the lanes with `mine`) within [t_lo,
+// cap]: bounds, walk and sort, over the warp's lists at smem[at]. A call of its own: the walk
+// and the passes over its list then keep their registers apart (in one piece, small changes
+// moved the kernel by 10%). Returns the number of leaves (packet_leaves) and the cap.
+struct LeafList {
+  int n;
+  float cap;
+  float area;  // of the group's tile of directions; +inf if its rays share no apex
+};
+__device__ __noinline__ LeafList list_leaves(const Node* nodes, const Record* recs, float3 o, float3 d, float3 apex,
+                                             bool mine, float t_lo, float cap, int limit, int at, int lane) {
+  extern __shared__ int smem[];
+  int* walk = smem + at;
+  uint64_t* cand = reinterpret_cast<uint64_t*>(walk + 2 * kWalkCap);
+  PacketTile* tile = reinterpret_cast<PacketTile*>(walk + 2 * kWalkCap + 2 * kCandCap + kStateWords * 32);
+  Ray ray;
+  ray.o = o;
+  ray.d = d;
+  ray.apex = apex;
+  float area;
+  const PacketBounds P = packet_bounds(ray, make_slab(ray), mine, tile, lane, &area);
+  const bool cull = area < INFINITY;
+  const int n = packet_leaves(nodes, recs, P, tile, cull, t_lo, &cap, cull ? limit : kStageLeaves, walk, cand, lane);
+  if (n > 0) sort_keys(cand, n, lane);
+  return LeafList{n, cap, area};
 }
 
-// The frustum phase of a warp's packet. Returns whether this lane's ray still needs rounds
-// (L then holds its state after its last integrated event, L.lower that event's key).
-template <int KBUF, int DEG>
-__device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx& C, const Ray& ray, const float* B,
-                                              int bs, int64_t slot, int64_t r, int* wsm, int lane, bool act,
-                                              RayLoop& L) {
-  constexpr int FBUF = frustum_buffer(KBUF);
-  if (!__any_sync(kFull, act)) return act;
-  const RaySlab sl = make_slab(ray);
-  float cap = fminf(C.tmax, kSentinel);
-  // With a depth hint the walk covers t up to the packet's largest guessed stopping t (plus
-  // 5%): events up to there are integrated here, the rounds continue any ray that goes on.
-  // A poor guess costs time, never correctness.
-  float t_final = INFINITY;
-  if (C.depth_hint) {
-    const float h = warp_max(act ? C.depth_hint[r] : -INFINITY);
-    if (h > 0.f && 1.05f * h + 1e-3f < cap) cap = t_final = 1.05f * h + 1e-3f;
-  }
-  const PacketBounds P = packet_bounds(ray, sl, act);
-  int* front = wsm + kStackDepth;
-  uint64_t* cand = reinterpret_cast<uint64_t*>(front + 2 * kFrontierCap);
-  const int nc = packet_leaves(sc.nodes, P, cap, front, cand, lane);
-  if (nc < 0) return act;  // lists too long for shared memory: the rounds trace the packet
-  sort_keys(cand, nc, lane);
-  uint64_t buf[FBUF];
+// Events that the frustum phase has put in order but not yet integrated: a ring per lane in
+// shared memory (over the walk's stack, which is done by then). The ordering step keeps only
+// the density and optical-depth sums that decide when a ray ends; colour, distortion and the
+// rest of the state stay in shared memory and take their events kRingBurst at a time, when
+// some lane's ring is full, so that most lanes integrate together.
+constexpr int kRing = kWalkCap / 32;  // events per lane
+constexpr int kRingBurst = kRing / 2;
+static_assert(kRing * 32 == kWalkCap, "the ring takes the walk's stack");
+
+struct Ring {
+  uint64_t* ev;  // [kRing][32]
+  float* st;     // [kStateWords][32]
+  int head, n;   // this lane's first event and their number
+};
+
+__device__ __forceinline__ void ring_state_store(float* st, int lane, const State& s) {
+  const float v[13] = {s.dist_x, s.dist_y, s.cum_x, s.cum_y, s.t, s.drgb.x, s.drgb.y, s.drgb.z, s.drgb.w,
+                       s.logT,   s.C.x,    s.C.y,   s.C.z};
 #pragma unroll
-  for (int i = 0; i < FBUF; ++i) buf[i] = kEmptyKey;
-  bool live = act;  // still integrating in this phase
-  for (int ci = 0;; ++ci) {
-    // every 32 leaves, the lanes start the loads of the next 32 records into L1 (one each),
-    // so the broadcast record loads of the loop below rarely wait on L2
-    if ((ci & 31) == 0 && ci + lane < nc)
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(sc.recs + int(uint32_t(cand[ci + lane]))));
-    const uint64_t ck = ci < nc ? cand[ci] : kEmptyKey;
-    const float T = ci < nc ? key_t(ck) : t_final;
-    // events below T are final: no leaf still to come has an event before T
-    while (live && buf[0] != kEmptyKey && key_t(buf[0]) < T) {
+  for (int i = 0; i < 13; ++i) st[32 * i + lane] = v[i];
+}
+__device__ __forceinline__ State ring_state_load(const float* st, int lane) {
+  float v[13];
+#pragma unroll
+  for (int i = 0; i < 13; ++i) v[i] = st[32 * i + lane];
+  State s;
+  s.dist_x = v[0];
+  s.dist_y = v[1];
+  s.cum_x = v[2];
+  s.cum_y = v[3];
+  s.t = v[4];
+  s.drgb = make_float4(v[5], v[6], v[7], v[8]);
+  s.logT = v[9];
+  s.C = make_float3(v[10], v[11], v[12]);
+  return s;
+}
+
+// Control point of an event: +-density and +-density * colour.
+template <int DEG>
+__device__ __forceinline__ float4 event_dirac(const SceneRef& sc, const float* B, int bs, uint32_t id) {
+  const int j = int(id >> 1);
+  const float4 r3 = __ldg(&sc.recs[j].r3);
+  const float3 c = DEG == 0 ? dc_colour(r3) : sh_colour<DEG>(sc.features + int64_t(j) * feat_stride(sc.K), B, bs);
+  const float dh = (id & 1u) ? -r3.x : r3.x;
+  return make_float4(dh, dh * c.x, dh * c.y, dh * c.z);
+}
+
+// Integrates up to `most` of each lane's waiting events.
+template <int DEG>
+__device__ __forceinline__ void ring_integrate(const SceneRef& sc, const float* B, int bs, Ring& q, int lane,
+                                               int most) {
+  const int n = min(q.n, most);
+  if (n > 0) {
+    State s = ring_state_load(q.st, lane);
+    uint32_t id = 0;
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+      const uint64_t k = q.ev[((q.head + i) & (kRing - 1)) * 32 + lane];
+      id = uint32_t(k);
+      update(s, key_t(k), event_dirac<DEG>(sc, B, bs, id));
+    }
+    ring_state_store(q.st, lane, s);
+    q.st[32 * 13 + lane] = __uint_as_float(id);
+    q.head += n;
+    q.n -= n;
+  }
+  __syncwarp();
+}
+
+// The entry root of ellipsoid j; a call, since only exits beyond tmax need it.
+__device__ __noinline__ float entry_time(const Record* recs, int j, float3 o, float3 d) {
+  Ray ray;
+  ray.o = o;
+  ray.d = d;
+  HitT H;
+  intersect(load_record(recs, j), ray, H);
+  return H.t0;
+}
+
+// Takes every lane's next events, all before T: in order, under the reference's round rules
+// (as consume_event), into the event log and the lane's ring. Clears live and act of a
+// lane whose ray ends. drain: also integrates what is left in the rings.
+template <int FBUF, int DEG>
+__device__ __forceinline__ void order_events(const SceneRef& sc, const TraceCtx& C, const Ray& ray, const float* B,
+                                             int bs, int64_t slot, int lane, uint64_t T, uint64_t (&buf)[FBUF],
+                                             Ring& q, RayLoop& L, float& sigma, float& t_last, float& depth,
+                                             bool& live, bool& act, bool drain) {
+#pragma unroll 1
+  for (;;) {
+    const bool want = live && buf[0] < T;
+    const bool any = __any_sync(kFull, want);
+    // the one place that integrates: a full ring, or the end of a pass with events waiting
+    if (__any_sync(kFull, any ? want && q.n == kRing : drain && q.n > 0))
+      ring_integrate<DEG>(sc, B, bs, q, lane, kRingBurst);
+    else if (!any)
+      break;
+    if (want) {
       const uint64_t k = buf[0];
 #pragma unroll
       for (int i = 0; i < FBUF - 1; ++i) buf[i] = buf[i + 1];
       buf[FBUF - 1] = kEmptyKey;
       L.lower = k;
-      if (consume_event<DEG>(sc, C, ray, B, bs, slot, k, L.s, L.last_dirac, L.iters, L.s16, L.cnt16, L.status)) {
-        live = false;
-        act = false;  // finished
+      const float t = key_t(k);
+      const int j = key_pos(k), ex = key_exit(k);
+      bool take = t > L.s16;
+      bool done = false;
+      if (take && t > kSentinel) {
+        take = false;
+        done = true;
       }
-    }
-    if (ci >= nc) break;
-    if (!__any_sync(kFull, live)) break;
-    if (live) {
-      const int j = int(uint32_t(ck));
-      const Record R = load_record(sc.recs, j);
-      HitT H;
-      if (intersect(R, ray, H)) {
-        const bool in0 = H.t0 > L.s16 && H.t0 <= C.tmax;
-        const bool in1 = H.t1 > L.s16 && (H.t1 <= C.tmax || in0);
-        // a full buffer cannot take another event: stop here, the rounds continue the ray
-        if ((in0 || in1) && buf[FBUF - (in0 && in1 ? 2 : 1)] != kEmptyKey) {
-          live = false;
-        } else {
-          if (in0) buf_insert(buf, event_key(H.t0, j, 0));
-          if (in1) buf_insert(buf, event_key(H.t1, j, 1));
+      if (take && ex && t > C.tmax) {
+        const float t0 = entry_time(sc.recs, j, ray.o, ray.d);
+        take = t0 > L.s16 && t0 <= C.tmax;
+      }
+      if (take) {
+        const float rho = __ldg(&sc.recs[j].r3.x);
+        const float area = fmaxf(sigma * fmaxf(t - t_last, 0.f), 0.f);
+        depth = fmaxf(area + depth, 0.f);
+        sigma = sigma + (ex ? -rho : rho);
+        t_last = t;
+        q.ev[((q.head + q.n) & (kRing - 1)) * 32 + lane] = k;
+        ++q.n;
+        if (C.out.event_log) {
+          if (L.iters < C.out.log_cap)
+            C.out.event_log[slot * int64_t(C.out.log_cap) + L.iters] = 2 * j + (ex ? 0 : 1);
+          else
+            L.status |= EVER_STATUS_LOG_OVERFLOW;
         }
+        if (C.out.touch_count) atomicAdd(C.out.touch_count + __ldg(sc.order + j), 1);
+        ++L.iters;
+        if (++L.cnt16 == kRefRound) {
+          L.s16 = t;
+          L.cnt16 = 0;
+        }
+        done = !(depth < kLogCutoff && L.iters < C.max_iters);
       }
+      if (done) live = act = false;
     }
   }
-  // all leaves taken and every event integrated: nothing is left on a lane still active,
-  // unless the walk stopped short of the scene (depth hint)
-  if (live && t_final == INFINITY) act = false;
+}
+
+// The lanes of `todo` to trace as one group: all of them, or those before a gap in the order
+// of directions more than 12 times the usual one (a launch order that leaves one patch of
+// directions for a distant one inside the packet: the union of both would meet far too much).
+__device__ __forceinline__ unsigned pick_group(const Ray& ray, unsigned todo, int lane) {
+  const float px = __shfl_up_sync(kFull, ray.d.x, 1), py = __shfl_up_sync(kFull, ray.d.y, 1),
+              pz = __shfl_up_sync(kFull, ray.d.z, 1);
+  const bool pair = lane > 0 && ((todo >> (lane - 1)) & 3u) == 3u;
+  const float gap = pair ? fabsf(ray.d.x - px) + fabsf(ray.d.y - py) + fabsf(ray.d.z - pz) : 0.f;
+  const float most = warp_max(gap);
+  float sum = gap;
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(kFull, sum, m);
+  // the mean of the gaps up to the mean of all: what neighbours are apart
+  const bool small = pair && gap * float(__popc(todo & (todo >> 1))) <= sum;
+  float usual = small ? gap : 0.f;
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1) usual += __shfl_xor_sync(kFull, usual, m);
+  const int n = __popc(__ballot_sync(kFull, small));
+  if (!(most * float(n) > 12.f * usual)) return todo;
+  const int at = __ffs(__ballot_sync(kFull, pair && gap == most)) - 1;
+  const unsigned before = todo & ((1u << at) - 1u);
+  return before ? before : todo;
+}
+
+// Whether the rays of `todo` come in no order: 16 or more, neighbours apart by more than a
+// fifth of the whole range of directions or of origins (random points: a third; runs of a
+// curve or a tile: a tenth to a sixth). No common list serves them.
+__device__ __forceinline__ bool no_order(const Ray& ray, unsigned todo, int lane) {
+  const bool part = todo >> lane & 1u, pair = lane > 0 && ((todo >> (lane - 1)) & 3u) == 3u;
+  const int pairs = __popc(todo & (todo >> 1));
+  const float v[6] = {ray.d.x, ray.d.y, ray.d.z, ray.o.x, ray.o.y, ray.o.z};
+  bool out = false;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    float gap = 0.f, range = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float x = h ? v[3 + a] : v[a], y = __shfl_up_sync(kFull, x, 1);
+      gap += pair ? fabsf(x - y) : 0.f;
+      range += warp_max(part ? x : -INFINITY) - warp_min(part ? x : INFINITY);
+    }
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) gap += __shfl_xor_sync(kFull, gap, m);
+    out = out || gap > 0.2f * range * float(pairs);
+  }
+  return out && pairs >= 15;
+}
+
+// The lower half of a group's lanes.
+__device__ __forceinline__ unsigned half_group(unsigned grp, int lane) {
+  const bool low = (grp >> lane & 1u) && 2 * __popc(grp & ((1u << lane) - 1u)) < __popc(grp);
+  return __ballot_sync(kFull, low);
+}
+
+// The frustum phase of a warp's packet, in stages over t: a stage lists the leaves of the
+// next t range (the whole scene, unless they do not fit or a depth hint ends it early) and
+// takes every event in it. The packet is traced as one group of lanes, or in several where
+// its directions leave a gap or a stage's leaves are met by few of its lanes. Returns whether
+// this lane's ray still needs rounds (L then holds its state after its last integrated event,
+// L.lower that event's key): only where more leaves than the list holds reach over one t.
+template <int KBUF, int DEG>
+__device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx& C, const Ray& ray, const float* B,
+                                              int bs, int64_t slot, int64_t r, int at, int lane, bool act,
+                                              RayLoop& L) {
+  extern __shared__ int smem[];
+  constexpr int FBUF = frustum_buffer(KBUF);
+  if (!__any_sync(kFull, act)) return act;
+  const float cap_all = fminf(C.tmax, kSentinel);
+  int* walk = smem + at;  // the warp's lists
+  uint64_t* cand = reinterpret_cast<uint64_t*>(walk + 2 * kWalkCap);
+  Ring q{reinterpret_cast<uint64_t*>(walk), reinterpret_cast<float*>(cand + kCandCap), 0, 0};
+  ring_state_store(q.st, lane, L.s);
+  // the ordering step's own copy of what decides the ray's end
+  float sigma = L.s.drgb.x, t_last = L.s.t, depth = L.s.logT;
+  const int first = L.iters;
+  float t_done = 0.f;  // every event of this lane's ray before it has been taken
+  float whole = INFINITY;  // tile area of the group a half was taken from
+  unsigned todo = __ballot_sync(kFull, act), grp = pick_group(ray, todo, lane);
+  if (grp == todo && no_order(ray, todo, lane)) return act;
+#pragma unroll 1
+  for (int stage = 0; todo && stage < kMaxStages; ++stage) {
+    const bool mine = grp >> lane & 1u;
+    const float t_lo = warp_min(mine ? t_done : INFINITY);
+    float cap = cap_all;
+    // With a depth hint a group's first stage covers t up to its largest guessed stopping t
+    // (plus 5%). A poor guess costs time, never correctness.
+    if (C.depth_hint && t_lo == 0.f) {
+      const float h = warp_max(mine ? C.depth_hint[r] : -INFINITY);
+      if (h > 0.f && 1.05f * h + 1e-3f < cap) cap = 1.05f * h + 1e-3f;
+    }
+    const LeafList list = list_leaves(sc.nodes, sc.recs, ray.o, ray.d, ray.apex, mine, t_lo, cap,
+                                      t_lo == 0.f ? kFirstLeaves : kStageLeaves, at, lane);
+    const int nc = list.n;
+    const bool cut = list.cap < cap;
+    cap = list.cap;
+    // half a group's lanes cover as much as all did: directions in no order, for the rounds
+    if (list.area > 0.7f * whole) break;
+    whole = INFINITY;
+    if (nc < 0) {  // does not fit: fewer rays at a time, or the rounds
+      if (__popc(grp) > 1 && list.area < INFINITY) {
+        whole = list.area;
+        grp = half_group(grp, lane);
+      } else {
+        todo &= ~grp;
+        grp = pick_group(ray, todo, lane);
+      }
+      continue;
+    }
+    // events from `end` on belong to the next stage
+    const uint64_t end = uint64_t(cap < cap_all ? __float_as_uint(cap) : 0x7f800000u) << 32;
+    // Passes over the list: one, unless a lane's buffer overflows. It then keeps its smallest
+    // events and takes those; the events from `over` (the smallest it dropped) on are
+    // collected again by another pass.
+    bool pending = mine;
+    int hits = 0;
+#pragma unroll 1
+    do {
+      uint64_t buf[FBUF];
+#pragma unroll
+      for (int i = 0; i < FBUF; ++i) buf[i] = kEmptyKey;
+      uint64_t over = kEmptyKey;
+      bool live = pending;
+#pragma unroll 1
+      for (int ci = 0;; ++ci) {
+        // every 32 leaves, the lanes start the loads of the next 32 records into L1 (one each),
+        // so the broadcast record loads of the loop below rarely wait on L2
+        if ((ci & 31) == 0 && ci + lane < nc)
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(sc.recs + int(uint32_t(cand[ci + lane]))));
+        const uint64_t ck = ci < nc ? cand[ci] : kEmptyKey;
+        // events below T are final: no leaf still to come has an event before T
+        const uint64_t T = ci < nc ? (ck & ~uint64_t(0xffffffffu)) : end;
+        const bool stop = ci >= nc || !__any_sync(kFull, live);
+        // ordering waits for a few leaves' events, so that more lanes take part in it
+        if (stop || (ci & (kHold - 1)) == 0 || __any_sync(kFull, live && buf[FBUF - 2] != kEmptyKey))
+          order_events<FBUF, DEG>(sc, C, ray, B, bs, slot, lane, T, buf, q, L, sigma, t_last, depth, live, act,
+                                  stop);
+        if (stop) break;
+        live = live && T < over;
+        // few buffered events in every lane (nearly always): an insertion moves only the first
+        const bool low = !__any_sync(kFull, live && buf[kLowEvents] != kEmptyKey);
+        if (live) {
+          const int j = int(uint32_t(ck));
+          const Record R = load_record(sc.recs, j);
+          HitT H;
+          if (intersect(R, ray, H)) {
+            ++hits;
+            const bool in0 = H.t0 > L.s16 && H.t0 <= C.tmax;
+            const bool in1 = H.t1 > L.s16 && (H.t1 <= C.tmax || in0);
+            uint64_t e0 = event_key(H.t0, j, 0), e1 = event_key(H.t1, j, 1);
+            e0 = in0 && e0 > L.lower && e0 < over ? e0 : kEmptyKey;
+            e1 = in1 && e1 > L.lower && e1 < over ? e1 : kEmptyKey;
+            if (low) {
+              buf_insert_low<kLowEvents + 2>(buf, e0);
+              buf_insert_low<kLowEvents + 2>(buf, e1);
+            } else {
+              e0 = buf_insert_low<FBUF>(buf, e0);
+              e1 = e1 < e0 ? buf_insert_low<FBUF>(buf, e1) : e1;
+              over = min(over, min(e0, e1));
+            }
+          }
+        }
+      }
+      pending = pending && act && over < end;
+    } while (__any_sync(kFull, pending));
+    if (mine) {
+      t_done = cap;
+      if (cap >= cap_all) act = false;
+    }
+    const unsigned left = __ballot_sync(kFull, act);
+    // a list that had to be cut short and that fewer than one lane in 32 met on average: the
+    // group is too wide
+    const bool wide = __reduce_add_sync(kFull, hits) * 32 < nc * __popc(grp);
+    todo &= left;
+    grp &= left;
+    if (cut && !(list.area < INFINITY)) {  // no apex to halve the directions around: the rounds
+      todo &= ~grp;
+      grp = 0;
+    }
+    if (!grp) {
+      grp = pick_group(ray, todo, lane);
+    } else if (cut && wide && __popc(grp) > 1) {
+      whole = list.area;
+      grp = half_group(grp, lane);
+    }
+  }
+  L.s = ring_state_load(q.st, lane);
+  if (L.iters > first) L.last_dirac = event_dirac<DEG>(sc, B, bs, __float_as_uint(q.st[32 * 13 + lane]));
+  __syncwarp();
   return act;
 }
 
-// One warp traces one packet of up to 32 rays against one scene (lanes with valid=false
-// only take part in the warp-wide votes).
+// The rounds that finish what the frustum phase leaves: rarely anything, so they are a call
+// (inlined, they would cost the whole kernel registers), with its arguments in local memory.
+struct RoundsCall {
+  SceneRef sc;
+  TraceCtx C;
+  Ray ray;
+  const float* B;
+  int bs, lane;
+  int64_t slot;
+  int* wstack;
+  bool act;
+  RayLoop L;
+};
 template <int KBUF, int DEG>
+__device__ __noinline__ void rounds_call(RoundsCall* a) {
+  RayLoop L = a->L;
+  run_rounds<KBUF, DEG>(a->sc, a->C, a->ray, a->B, a->bs, a->slot, a->wstack, a->lane, a->act, L, INT_MAX);
+  a->L = L;
+}
+
+// One warp traces one packet of up to 32 rays against one scene (lanes with valid=false
+// only take part in the warp-wide votes). FRUSTUM: the frustum phase, else rounds only.
+template <int KBUF, int DEG, bool FRUSTUM>
 __device__ __forceinline__ void trace_packet(const SceneRef& sc, const TraceCtx& C, const Ray& ray, int64_t r,
                                              bool valid, int64_t slot, int* wstack, float* B, int bs, int lane) {
   store_basis<DEG>(ray, B, bs);
   RayLoop L = start_ray<DEG>(sc, ray, valid, wstack, C.depth, B, bs, lane);
   bool act = valid && C.max_iters > 0 && sc.N > 0;
-  if (C.frustum) act = frustum_phase<KBUF, DEG>(sc, C, ray, B, bs, slot, r, wstack, lane, act, L);
-  run_rounds<KBUF, DEG>(sc, C, ray, B, bs, slot, wstack, lane, act, L, INT_MAX);
+  if (FRUSTUM) {
+    act = frustum_phase<KBUF, DEG>(sc, C, ray, B, bs, slot, r, int(threadIdx.x >> 5) * kWarpInts, lane, act, L);
+    if (__any_sync(kFull, act)) {
+      RoundsCall a{sc, C, ray, B, bs, lane, slot, wstack, act, L};
+      rounds_call<KBUF, DEG>(&a);
+      L = a.L;
+    }
+  } else {
+    run_rounds<KBUF, DEG>(sc, C, ray, B, bs, slot, wstack, lane, act, L, INT_MAX);
+  }
   if (valid) write_outputs(C.out, r, L.s, L.last_dirac, L.iters, L.status);
   __syncwarp();
 }
@@ -878,26 +1407,27 @@ __device__ __forceinline__ RayLoop resume_ray(const EverForwardOut& out, int64_t
   return L;
 }
 
-// Resident blocks per SM that the register budget of the packet kernels targets: 20
-// warps per SM for blocks of 64 and 128 threads (96 registers; the traversal is
-// latency-bound, so the extra warps pay for a few spilled bytes), 16 for 256 threads.
-template <int BLOCK>
+// Resident blocks per SM that the register budget of the packet kernels targets: 16 warps
+// (128 registers) with the frustum phase, which is bound by instructions and not by latency
+// (3.6 ms at 1M ellipsoids / 1080p; 20 warps: 3.8, 24: 3.9 ms, with spills); 20 warps (96
+// registers) for the rounds, whose traversal is latency-bound.
+template <int BLOCK, bool FRUSTUM = true>
 struct FwdMinBlocks {
-  static constexpr int value = BLOCK == 256 ? 2 : 640 / BLOCK;
+  static constexpr int value = BLOCK == 256 ? 2 : (FRUSTUM ? 512 : 640) / BLOCK;
 };
 
 template <int KBUF, int DEG, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK>::value) k_trace_fwd_packet(const FwdParams P) {
   extern __shared__ int smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int* wstack = smem + warp * kWarpInts;  // stack, then the frustum phase's lists
+  int* wstack = smem + warp * kWarpInts;  // traversal stack, and the frustum phase's lists over it
   float* B = reinterpret_cast<float*>(smem + (blockDim.x / 32) * kWarpInts) + tid;  // B[k * blockDim.x]
-  const int64_t gi = int64_t(blockIdx.x) * blockDim.x + tid;
-  const bool valid = gi < P.R;  // every lane stays for the warp-wide ballots
+  const int64_t gi = (int64_t(blockIdx.x) * (blockDim.x / 32) + warp) * P.lanes + lane;
+  const bool valid = lane < P.lanes && gi < P.R;  // every lane stays for the warp-wide ballots
   const int64_t r = valid ? (P.ray_order ? int64_t(P.ray_order[gi]) : gi) : 0;
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.frustum != 0, P.stack_depth, P.depth_hint};
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
   const Ray ray = load_ray(P.rayo, P.rayd, r, P.tmin);
-  trace_packet<KBUF, DEG>(scene_of(P), C, ray, r, valid, gi, wstack, B, blockDim.x, lane);
+  trace_packet<KBUF, DEG, true>(scene_of(P), C, ray, r, valid, gi, wstack, B, blockDim.x, lane);
 }
 
 // Regrouped forward, one pass. PASS 0 takes every slot in order and runs the first gather
@@ -917,13 +1447,13 @@ struct PassCamera {
 };
 
 template <int KBUF, int DEG, int BLOCK, int PASS, bool CAM>
-__global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK>::value)
+__global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK, false>::value)
     k_trace_fwd_pass(const FwdParams P, const int32_t* __restrict__ list, const uint32_t* __restrict__ count,
                      uint32_t* __restrict__ mask, int64_t split_min, const PassCamera Q) {
   extern __shared__ int smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int* wstack = smem + warp * kWarpInts;  // stack, then the frustum phase's lists
-  float* B = reinterpret_cast<float*>(smem + (blockDim.x / 32) * kWarpInts) + tid;
+  int* wstack = smem + warp * kStackDepth;
+  float* B = reinterpret_cast<float*>(smem + (blockDim.x / 32) * kStackDepth) + tid;
   const int64_t gi = int64_t(blockIdx.x) * blockDim.x + tid;  // slot (PASS 0) or list position
   const int64_t slots = CAM ? Q.num_slots : P.R;
   const int64_t n = PASS == 0 ? slots : int64_t(*count);
@@ -939,7 +1469,7 @@ __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK>::value)
   }
   if (!valid) r = 0;
   const SceneRef sc = scene_of(P);
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.frustum != 0, P.stack_depth, P.depth_hint};
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
   Ray ray;
   if (CAM) {
     float3 ro, rd;
@@ -954,16 +1484,13 @@ __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK>::value)
   if (PASS == 0) {
     L = start_ray<DEG>(sc, ray, valid, wstack, C.depth, B, blockDim.x, lane);
     act = valid && C.max_iters > 0 && sc.N > 0;
-    if (C.frustum) act = frustum_phase<KBUF, DEG>(sc, C, ray, B, blockDim.x, slot, r, wstack, lane, act, L);
   } else {
     if (valid) L = resume_ray(P.out, r);
     act = valid;
   }
   const bool last = PASS == 2 || n < split_min;
-  // after the frustum phase, pass 0 hands its few unfinished rays on without a round
-  const int rounds = last ? INT_MAX : (PASS == 0 && C.frustum ? 0 : 1);
-  act = run_rounds<KBUF, DEG>(sc, C, ray, B, blockDim.x, slot, wstack, lane, act, L, rounds);
-  if (PASS < 2) {
+  act = run_rounds<KBUF, DEG>(sc, C, ray, B, blockDim.x, slot, wstack, lane, act, L, last ? INT_MAX : 1);
+  if (PASS < 2 && mask) {
     const unsigned m = __ballot_sync(kFull, act);
     if (lane == 0) mask[gi >> 5] = m;
   }
@@ -984,50 +1511,54 @@ __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK>::value)
                        int64_t num_slots) {
   extern __shared__ int smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int* wstack = smem + warp * kWarpInts;  // stack, then the frustum phase's lists
+  int* wstack = smem + warp * kWarpInts;  // traversal stack, and the frustum phase's lists over it
   float* B = reinterpret_cast<float*>(smem + (blockDim.x / 32) * kWarpInts) + tid;
-  const int64_t gi = int64_t(blockIdx.x) * blockDim.x + tid;
-  const int64_t p = gi < num_slots ? camera_slot_pixel(cam, gi) : -1;
+  const int64_t gi = (int64_t(blockIdx.x) * (blockDim.x / 32) + warp) * P.lanes + lane;
+  const int64_t p = lane < P.lanes && gi < num_slots ? camera_slot_pixel(cam, gi) : -1;
   const bool valid = p >= 0;
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.frustum != 0, P.stack_depth, P.depth_hint};
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
   float3 ro, rd;
   camera_ray(cam, jitter, valid ? p : 0, ro, rd);
   const Ray ray = make_ray(ro, rd, P.tmin);
-  trace_packet<KBUF, DEG>(scene_of(P), C, ray, valid ? p : 0, valid, gi, wstack, B, blockDim.x, lane);
+  trace_packet<KBUF, DEG, true>(scene_of(P), C, ray, valid ? p : 0, valid, gi, wstack, B, blockDim.x, lane);
 }
 
 // Persistent batched forward: warps take 32-slot packets from a device counter until
 // all views are done. Each packet lies inside one view, hence one scene.
-template <int KBUF, int DEG, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK>::value) k_trace_fwd_batched(const BatchFwdParams P) {
+template <int KBUF, int DEG, int BLOCK, bool FRUSTUM>
+__global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK, FRUSTUM>::value)
+    k_trace_fwd_batched(const BatchFwdParams P) {
   extern __shared__ int smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int* wstack = smem + warp * kWarpInts;  // stack, then the frustum phase's lists
-  float* B = reinterpret_cast<float*>(smem + (blockDim.x / 32) * kWarpInts) + tid;
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.frustum != 0, P.stack_depth, nullptr};
-  const int64_t num_packets = P.num_slots / 32;
+  constexpr int kInts = FRUSTUM ? kWarpInts : kStackDepth;  // traversal stack, and the frustum phase's lists over it
+  int* wstack = smem + warp * kInts;
+  float* B = reinterpret_cast<float*>(smem + (blockDim.x / 32) * kInts) + tid;
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, nullptr};
+  const int lanes = FRUSTUM ? P.lanes : 32;  // a divisor of 32: a packet never mixes views
+  const int64_t num_packets = P.num_slots / lanes;
   for (;;) {
     unsigned int pk = 0;
     if (lane == 0) pk = atomicAdd(P.work_counter, 1u);
     pk = __shfl_sync(kFull, pk, 0);
     if (int64_t(pk) >= num_packets) break;
-    const int64_t slot = int64_t(pk) * 32 + lane;
+    const int64_t first = int64_t(pk) * lanes, slot = first + lane;
     int v = 0;  // the view holding this packet (few views: linear scan, warp-uniform)
-    while (v + 1 < P.num_views && P.views[v + 1].slot_offset <= int64_t(pk) * 32) ++v;
+    while (v + 1 < P.num_views && P.views[v + 1].slot_offset <= first) ++v;
     const BatchScene bs_ = P.scenes[P.views[v].scene];
     const SceneRef sc{reinterpret_cast<const Node*>(bs_.nodes), reinterpret_cast<const Record*>(bs_.records),
                       bs_.features, bs_.order, bs_.N, bs_.K};
-    const int32_t r = P.slot_ray[slot];
+    const int32_t r = lane < lanes ? P.slot_ray[slot] : -1;
     const Ray ray = load_ray(P.rayo, P.rayd, r >= 0 ? r : 0, P.tmin);
-    trace_packet<KBUF, DEG>(sc, C, ray, r, r >= 0, slot, wstack, B, blockDim.x, lane);
+    trace_packet<KBUF, DEG, FRUSTUM>(sc, C, ray, r, r >= 0, slot, wstack, B, blockDim.x, lane);
   }
 }
 
-// Dynamic shared memory of a packet kernel: per warp its stack and frustum-phase lists,
-// per thread the SH basis of its ray.
+// Dynamic shared memory of a packet kernel: per warp its frustum-phase lists (or, for rounds
+// only, its traversal stack), per thread the SH basis of its ray.
 template <int DEG>
-size_t packet_smem(int block) {
-  return size_t(kWarpInts) * (block / 32) * sizeof(int) + size_t((DEG + 1) * (DEG + 1)) * block * sizeof(float);
+size_t packet_smem(int block, bool frustum = true) {
+  return size_t(frustum ? kWarpInts : kStackDepth) * (block / 32) * sizeof(int) +
+         size_t((DEG + 1) * (DEG + 1)) * block * sizeof(float);
 }
 
 // Dynamic shared memory above the 48 KB default needs the kernel's opt-in.
@@ -1037,15 +1568,51 @@ cudaError_t prepare(Kern kern, size_t smem) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
 }
 
+// Rays per packet. A launch that leaves warps idle takes fewer rays in each: a warp's time is
+// the chain of its packet's leaves and events, and narrower packets have fewer (kernel time
+// with 32 / 16 / 8 / 4 rays: 4,096 rays against 1,000 ellipsoids 115 / 71 / 55 / 50 us, 9,471
+// rays against 20,000 400 / 262 / 177 / 91 us). Halved while the launch then still fits the
+// resident warps (16 per SM); 4 rays at least (2: 82 us, the walk is repeated too often).
+inline int packet_lanes(int64_t rays) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int lanes = 32;
+  while (lanes > 4 && rays <= int64_t(sms) * 16 * (lanes / 2)) lanes /= 2;
+  return lanes;
+}
+
+// Gather rounds only, one pass that runs them all.
+template <int KBUF, int DEG, int BLOCK, bool CAM>
+cudaError_t launch_rounds_b(const FwdParams& P, const PassCamera& Q, cudaStream_t st) {
+  const int64_t n = CAM ? Q.num_slots : P.R;
+  const size_t smem = packet_smem<DEG>(BLOCK, false);
+  if (cudaError_t e_ = prepare(k_trace_fwd_pass<KBUF, DEG, BLOCK, 0, CAM>, smem)) return e_;
+  k_trace_fwd_pass<KBUF, DEG, BLOCK, 0, CAM>
+      <<<unsigned((n + BLOCK - 1) / BLOCK), BLOCK, smem, st>>>(P, nullptr, nullptr, nullptr, INT64_MAX, Q);
+  return cudaGetLastError();
+}
+template <int KBUF, int DEG, bool CAM>
+cudaError_t launch_rounds(const FwdParams& P, const PassCamera& Q, int block, cudaStream_t st) {
+  switch (block) {
+    case 64: return launch_rounds_b<KBUF, DEG, 64, CAM>(P, Q, st);
+    case 128: return launch_rounds_b<KBUF, DEG, 128, CAM>(P, Q, st);
+    default: return launch_rounds_b<KBUF, DEG, 256, CAM>(P, Q, st);
+  }
+}
+
 template <int KBUF, int DEG>
-cudaError_t launch_t(const FwdParams& P, int block, int traversal, cudaStream_t st) {
-  const int64_t grid = (P.R + block - 1) / block;
+cudaError_t launch_t(const FwdParams& P0, int block, int traversal, cudaStream_t st) {
+  FwdParams P = P0;
+  P.lanes = traversal == 0 ? packet_lanes(P.R) : 32;
+  const int64_t grid = (P.R + P.lanes * (block / 32) - 1) / (P.lanes * (block / 32));
   if (traversal == 1) {
     const size_t smem = size_t(kStackDepth) * block * (sizeof(int) + sizeof(float));
     auto kern = k_trace_fwd_ray<KBUF, DEG>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     kern<<<unsigned(grid), block, smem, st>>>(P);
+  } else if (traversal == 2) {
+    return launch_rounds<KBUF, DEG, false>(P, PassCamera{}, block, st);
   } else {
     const size_t smem = packet_smem<DEG>(block);
     switch (block) {
@@ -1083,7 +1650,7 @@ template <int KBUF, int DEG, int BLOCK, bool CAM>
 cudaError_t launch_regrouped_b(const FwdParams& P, const RegroupScratch& W, const PassCamera& Q, cudaStream_t st) {
   const int64_t n = CAM ? Q.num_slots : P.R;
   const unsigned grid = unsigned((n + BLOCK - 1) / BLOCK);
-  const size_t smem = packet_smem<DEG>(BLOCK);
+  const size_t smem = packet_smem<DEG>(BLOCK, false);
   if (cudaError_t e_ = prepare(k_trace_fwd_pass<KBUF, DEG, BLOCK, 0, CAM>, smem)) return e_;
   k_trace_fwd_pass<KBUF, DEG, BLOCK, 0, CAM><<<grid, BLOCK, smem, st>>>(P, nullptr, nullptr, W.mask0, W.split_min, Q);
   cudaError_t e = regroup_compact(W.mask0, nullptr, n, nullptr, W.offsets, W.list1, W.count1, st);
@@ -1131,10 +1698,13 @@ cudaError_t launch_regrouped_k(const FwdParams& P, const RegroupScratch& W, cons
 }
 
 template <int KBUF, int DEG>
-cudaError_t launch_camera_t(const FwdParams& P, const CameraParams& cam, const float* jitter, int block,
-                            cudaStream_t st) {
+cudaError_t launch_camera_t(const FwdParams& P0, const CameraParams& cam, const float* jitter, int block,
+                            bool frustum, cudaStream_t st) {
   const int64_t num_slots = camera_slots(cam);
-  const unsigned grid = unsigned((num_slots + block - 1) / block);
+  if (!frustum) return launch_rounds<KBUF, DEG, true>(P0, PassCamera{cam, jitter, num_slots}, block, st);
+  FwdParams P = P0;
+  P.lanes = packet_lanes(num_slots);
+  const unsigned grid = unsigned((num_slots + P.lanes * (block / 32) - 1) / (P.lanes * (block / 32)));
   const size_t smem = packet_smem<DEG>(block);
   switch (block) {
     case 64: {
@@ -1159,37 +1729,35 @@ cudaError_t launch_camera_t(const FwdParams& P, const CameraParams& cam, const f
 template <int KBUF>
 cudaError_t launch_camera_k(const FwdParams& P, const CameraParams& cam, const float* jitter, int deg, int block,
                             cudaStream_t st) {
+  const bool f = P.frustum != 0;
   switch (deg) {
-    case 0: return launch_camera_t<KBUF, 0>(P, cam, jitter, block, st);
-    case 1: return launch_camera_t<KBUF, 1>(P, cam, jitter, block, st);
-    case 2: return launch_camera_t<KBUF, 2>(P, cam, jitter, block, st);
-    default: return launch_camera_t<KBUF, 3>(P, cam, jitter, block, st);
+    case 0: return launch_camera_t<KBUF, 0>(P, cam, jitter, block, f, st);
+    case 1: return launch_camera_t<KBUF, 1>(P, cam, jitter, block, f, st);
+    case 2: return launch_camera_t<KBUF, 2>(P, cam, jitter, block, f, st);
+    default: return launch_camera_t<KBUF, 3>(P, cam, jitter, block, f, st);
   }
+}
+
+template <int KBUF, int DEG, int BLOCK, bool FRUSTUM>
+cudaError_t launch_batched_b(const BatchFwdParams& P0, cudaStream_t st) {
+  BatchFwdParams P = P0;
+  P.lanes = FRUSTUM ? packet_lanes(P.num_slots) : 32;
+  const size_t smem = packet_smem<DEG>(BLOCK, FRUSTUM);
+  if (cudaError_t e_ = prepare(k_trace_fwd_batched<KBUF, DEG, BLOCK, FRUSTUM>, smem)) return e_;
+  k_trace_fwd_batched<KBUF, DEG, BLOCK, FRUSTUM><<<P.grid, BLOCK, smem, st>>>(P);
+  return cudaGetLastError();
 }
 
 template <int KBUF, int DEG>
 cudaError_t launch_batched_t(const BatchFwdParams& P, int block, cudaStream_t st) {
-  const size_t smem = packet_smem<DEG>(block);
   cudaError_t e = cudaMemsetAsync(P.work_counter, 0, sizeof(unsigned int), st);
   if (e != cudaSuccess) return e;
+  const bool f = P.frustum != 0;
   switch (block) {
-    case 64: {
-      if (cudaError_t e_ = prepare(k_trace_fwd_batched<KBUF, DEG, 64>, smem)) return e_;
-      k_trace_fwd_batched<KBUF, DEG, 64><<<P.grid, 64, smem, st>>>(P);
-      break;
-    }
-    case 128: {
-      if (cudaError_t e_ = prepare(k_trace_fwd_batched<KBUF, DEG, 128>, smem)) return e_;
-      k_trace_fwd_batched<KBUF, DEG, 128><<<P.grid, 128, smem, st>>>(P);
-      break;
-    }
-    default: {
-      if (cudaError_t e_ = prepare(k_trace_fwd_batched<KBUF, DEG, 256>, smem)) return e_;
-      k_trace_fwd_batched<KBUF, DEG, 256><<<P.grid, 256, smem, st>>>(P);
-      break;
-    }
+    case 64: return f ? launch_batched_b<KBUF, DEG, 64, true>(P, st) : launch_batched_b<KBUF, DEG, 64, false>(P, st);
+    case 128: return f ? launch_batched_b<KBUF, DEG, 128, true>(P, st) : launch_batched_b<KBUF, DEG, 128, false>(P, st);
+    default: return f ? launch_batched_b<KBUF, DEG, 256, true>(P, st) : launch_batched_b<KBUF, DEG, 256, false>(P, st);
   }
-  return cudaGetLastError();
 }
 
 template <int KBUF>
