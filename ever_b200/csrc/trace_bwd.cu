@@ -820,20 +820,34 @@ __global__ void k_finalize_features(const int32_t* __restrict__ order, int64_t N
   }
 }
 
-// tri[i * R + ray] from log[slot * log_cap + i], ray = ray_order[slot] (or slot).
+// The events of one slot into tri[i * R + r], which the launcher has cleared: one thread per
+// slot, so that 32 neighbouring rays write their i-th events together. Bound by the clearing
+// (4 max_iters bytes a ray, 145 us of the 213 us at 979 x 546 rays and 400 iterations): few
+// entries hold an event, and one thread per entry, each with its own division and ray
+// lookup, took 838 us. vec: the log's rows are whole 16-byte groups.
+__device__ __forceinline__ void log_row_to_reference(const int32_t* __restrict__ order, const int32_t* __restrict__ row,
+                                                     int n, int64_t R, int64_t r, bool vec,
+                                                     int32_t* __restrict__ tri) {
+  auto original = [&](int32_t id) { return 2 * __ldg(order + (id >> 1)) + (id & 1); };
+  int i = 0;
+  if (vec) {
+    for (; i + 4 <= n; i += 4) {
+      const int4 id = *reinterpret_cast<const int4*>(row + i);
+      const int32_t v[4] = {original(id.x), original(id.y), original(id.z), original(id.w)};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) tri[(i + q) * R + r] = v[q];
+    }
+  }
+  for (; i < n; ++i) tri[i * R + r] = original(row[i]);
+}
+
 __global__ void k_log_to_reference(const int32_t* __restrict__ order, const int32_t* __restrict__ log, int log_cap,
                                    const int32_t* __restrict__ iters, int64_t R, const int32_t* __restrict__ ray_order,
-                                   int32_t* __restrict__ tri, int max_iters) {
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= R * int64_t(max_iters)) return;
-  const int64_t i = t / R, slot = t - i * R;
+                                   int32_t* __restrict__ tri, int max_iters, bool vec) {
+  const int64_t slot = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (slot >= R) return;
   const int64_t r = ray_order ? int64_t(ray_order[slot]) : slot;
-  int32_t v = 0;
-  if (i < iters[r] && i < log_cap) {
-    const int32_t id = log[slot * log_cap + i];
-    v = 2 * order[id >> 1] + (id & 1);
-  }
-  tri[i * R + r] = v;
+  log_row_to_reference(order, log + slot * log_cap, min(min(iters[r], log_cap), max_iters), R, r, vec, tri);
 }
 
 template <int DEG>
@@ -858,18 +872,17 @@ __global__ void k_camera_slot_pixels(const CameraParams cam, int64_t num_slots, 
 __global__ void k_camera_log_to_reference(const CameraParams cam, int64_t num_slots, const int32_t* __restrict__ order,
                                           const int32_t* __restrict__ log, int log_cap,
                                           const int32_t* __restrict__ iters, int32_t* __restrict__ tri,
-                                          int max_iters) {
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= num_slots * int64_t(max_iters)) return;
-  const int64_t i = t / num_slots, slot = t - i * num_slots;
+                                          int max_iters, bool vec) {
+  const int64_t slot = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (slot >= num_slots) return;
   const int64_t r = camera_slot_pixel(cam, slot);
   if (r < 0) return;
-  int32_t v = 0;
-  if (i < iters[r] && i < log_cap) {
-    const int32_t id = log[slot * log_cap + i];
-    v = 2 * order[id >> 1] + (id & 1);
-  }
-  tri[i * (int64_t(cam.width) * cam.height) + r] = v;
+  log_row_to_reference(order, log + slot * log_cap, min(min(iters[r], log_cap), max_iters),
+                       int64_t(cam.width) * cam.height, r, vec, tri);
+}
+
+inline bool log_rows_aligned(const int32_t* log, int log_cap) {
+  return log_cap % 4 == 0 && reinterpret_cast<uintptr_t>(log) % 16 == 0;
 }
 
 template <int DEG>
@@ -924,10 +937,12 @@ cudaError_t launch_camera_slot_pixels(const CameraParams& cam, int32_t* slot_pix
 cudaError_t launch_camera_log_to_reference(const CameraParams& cam, const int32_t* order, const int32_t* log,
                                            int log_cap, const int32_t* iters, int32_t* tri, int max_iters,
                                            cudaStream_t st) {
-  const int64_t n = camera_slots(cam) * int64_t(max_iters);
-  if (n == 0) return cudaSuccess;
-  k_camera_log_to_reference<<<unsigned((n + 255) / 256), 256, 0, st>>>(cam, camera_slots(cam), order, log, log_cap,
-                                                                       iters, tri, max_iters);
+  const int64_t S = camera_slots(cam);
+  if (S == 0 || max_iters <= 0) return cudaSuccess;
+  const cudaError_t e = cudaMemsetAsync(tri, 0, int64_t(cam.width) * cam.height * max_iters * sizeof(int32_t), st);
+  if (e != cudaSuccess) return e;
+  k_camera_log_to_reference<<<unsigned((S + 127) / 128), 128, 0, st>>>(cam, S, order, log, log_cap, iters, tri,
+                                                                      max_iters, log_rows_aligned(log, log_cap));
   return cudaGetLastError();
 }
 
@@ -944,10 +959,11 @@ cudaError_t launch_finalize(const FinalizeParams& P, cudaStream_t st) {
 
 cudaError_t launch_log_to_reference(const int32_t* order, const int32_t* log, int log_cap, const int32_t* iters,
                                     int64_t R, const int32_t* ray_order, int32_t* tri, int max_iters, cudaStream_t st) {
-  const int64_t total = R * int64_t(max_iters);
-  if (total == 0) return cudaSuccess;
-  k_log_to_reference<<<unsigned((total + 255) / 256), 256, 0, st>>>(order, log, log_cap, iters, R, ray_order, tri,
-                                                                    max_iters);
+  if (R == 0 || max_iters <= 0) return cudaSuccess;
+  const cudaError_t e = cudaMemsetAsync(tri, 0, R * max_iters * sizeof(int32_t), st);
+  if (e != cudaSuccess) return e;
+  k_log_to_reference<<<unsigned((R + 127) / 128), 128, 0, st>>>(order, log, log_cap, iters, R, ray_order, tri,
+                                                               max_iters, log_rows_aligned(log, log_cap));
   return cudaGetLastError();
 }
 
