@@ -55,11 +55,14 @@ __device__ __forceinline__ float tukey(float x) {
   const float xs = fabsf(x) / fmaxf(kTiny, pm1);
   return ((sgnf(x) * pm1) / p) * (powf(xs + 1.f, p) - 1.f);
 }
-__device__ __forceinline__ float dtukey(float x) {
+// tukey and its derivative.
+__device__ __forceinline__ void tukey_both(float x, float& v, float& dv) {
   const float p = -0.1f;
   const float pm1 = fabsf(p - 1.f);
-  const float xs = fabsf(x) / fmaxf(kTiny, pm1);
-  return sgnf(x) * sgnf(x) * powf(xs + 1.f, p - 1.f);
+  const float x1 = fabsf(x) / fmaxf(kTiny, pm1) + 1.f;
+  const float sg = sgnf(x);
+  v = ((sg * pm1) / p) * (powf(x1, p) - 1.f);
+  dv = sg * sg * powf(x1, p - 1.f);
 }
 
 // rotate_vector(v, q): rotation by the conjugate of q = (r,x,y,z), safe-math.slang:236-244.

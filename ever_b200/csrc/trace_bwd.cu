@@ -16,144 +16,143 @@ namespace ever {
 namespace {
 
 constexpr int kGeo = 16;  // per-ellipsoid accumulator: W (9), mean (3), density (1), pad (3)
-// Resident 256-thread blocks per SM: 24 warps at degree 0 (80 registers; 2.06 ms against
-// 2.25 ms with 16 warps at 1M / 1080p), 16 warps with SH colour, which needs more registers.
+// Resident 256-thread blocks per SM: 24 warps at degree 0 (80 registers; at 1M / 1080p 1.46 ms,
+// 1.80 ms with 32 warps), 16 warps with SH colour, which needs more registers. The kernel waits on
+// its scattered records and the L2 atomics (without the atomics it takes 1.0 ms); each term of
+// a step is evaluated once: the intersection, the weight and the power were evaluated two to
+// three times each, and the kernel took 1.82 ms.
 template <int DEG>
 constexpr int kBwdMinBlocks = DEG == 0 ? 3 : 2;
 
+// One event of the replay. Its hit point P and den = P . rdn carry what the root's
+// derivative needs, so that each event's intersection is evaluated once.
 struct Ctrl {
   float t;
-  float4 dirac;
+  float dh;  // +density at the entry, -density at the exit
   float3 c;
-  int j, entry;
+  float P[3];  // hit point in the ellipsoid's unit-sphere frame
+  float den;
+  int id;  // 2 * position + entry
 };
 
-struct FullHit {
-  float t0, t1;
-  float ocn[3], rdn[3];
-};
-
-__device__ __forceinline__ bool intersect_full(const Record& R, const Ray& ray, FullHit& H) {
+// The event's root exactly as intersect() computes it, and the hit point in the
+// cancellation-free form P = l +- (sqrt(h)/a) rdn with P . rdn = +-sqrt(h).
+__device__ __forceinline__ void ctrl_root(const Record& R, const Ray& ray, bool entry, Ctrl& k) {
   const float v0 = ray.o.x - R.r0.w, v1 = ray.o.y - R.r1.w, v2 = ray.o.z - R.r2.w;
   const float4 rows[3] = {R.r0, R.r1, R.r2};
+  float oc[3], rn[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    H.ocn[i] = fmaf(rows[i].z, v2, fmaf(rows[i].y, v1, rows[i].x * v0));
-    H.rdn[i] = fmaf(rows[i].z, ray.d.z, fmaf(rows[i].y, ray.d.y, rows[i].x * ray.d.x));
+    oc[i] = fmaf(rows[i].z, v2, fmaf(rows[i].y, v1, rows[i].x * v0));
+    rn[i] = fmaf(rows[i].z, ray.d.z, fmaf(rows[i].y, ray.d.y, rows[i].x * ray.d.x));
   }
-  HitT h;
-  const bool hit = intersect(R, ray, h);
-  H.t0 = h.t0;
-  H.t1 = h.t1;
-  return hit;
+  const float a = fmaf(rn[2], rn[2], fmaf(rn[1], rn[1], rn[0] * rn[0]));
+  const float bp = -fmaf(oc[2], rn[2], fmaf(oc[1], rn[1], oc[0] * rn[0]));
+  const float ba = bp / a;
+  float l[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) l[i] = fmaf(ba, rn[i], oc[i]);
+  const float ll = fmaf(l[2], l[2], fmaf(l[1], l[1], l[0] * l[0]));
+  const float h = a * (1.f - ll);
+  const float c = fmaf(oc[2], oc[2], fmaf(oc[1], oc[1], oc[0] * oc[0])) - 1.f;
+  const float sq = sqrtf(fmaxf(h, 0.f));
+  const float qq = bp > 0.f ? bp + sq : (bp < 0.f ? bp - sq : bp);
+  const float ra = c / qq, rb = qq / a;
+  k.t = entry ? fminf(ra, rb) : fmaxf(ra, rb);
+  k.den = entry ? -sq : sq;
+  const float f = k.den / a;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) k.P[i] = fmaf(f, rn[i], l[i]);
 }
 
 template <int DEG>
 __device__ __forceinline__ Ctrl load_ctrl(const Record* recs, const float* feats, int64_t fstride, const Ray& ray,
                                           const float* B, int id) {
-  Ctrl c;
-  c.j = id >> 1;
-  c.entry = id & 1;
-  const Record R = load_record(recs, c.j);
-  HitT H;
-  intersect(R, ray, H);
-  c.t = c.entry ? H.t0 : H.t1;
-  c.c = DEG == 0 ? dc_colour(R.r3) : sh_colour<DEG>(feats + c.j * fstride, B);
-  const float dh = c.entry ? R.r3.x : -R.r3.x;
-  c.dirac = make_float4(dh, dh * c.c.x, dh * c.c.y, dh * c.c.z);
-  return c;
+  Ctrl k;
+  k.id = id;
+  const int j = id >> 1;
+  const bool entry = id & 1;
+  const Record R = load_record(recs, j);
+  ctrl_root(R, ray, entry, k);
+  k.c = DEG == 0 ? dc_colour(R.r3) : sh_colour<DEG>(feats + j * fstride, B);
+  k.dh = entry ? R.r3.x : -R.r3.x;
+  return k;
 }
 
-// inverse_update_dual, spline-machine.slang:65-100.
-__device__ __forceinline__ State inverse_update(const State& n, float4 dirac_new, float t_old) {
-  State s;
-  const float dt = fmaxf(n.t - t_old, 0.f);
-  s.drgb = make_float4(n.drgb.x - dirac_new.x, n.drgb.y - dirac_new.y, n.drgb.z - dirac_new.z,
-                       n.drgb.w - dirac_new.w);
-  s.t = t_old;
-  const float area = fmaxf(s.drgb.x * dt, 0.f);
-  const float rgb0 = safe_div(s.drgb.y, s.drgb.x), rgb1 = safe_div(s.drgb.z, s.drgb.x),
-              rgb2 = safe_div(s.drgb.w, s.drgb.x);
-  s.logT = fmaxf(n.logT - area, 0.f);
-  const float w = clampf((1.f - safe_exp(-area)) * safe_exp(-s.logT), 0.f, 1.f);
-  s.C = make_float3(n.C.x - w * rgb0, n.C.y - w * rgb1, n.C.z - w * rgb2);
-  const float m = tukey(((n.t + s.t) * 0.5f) * 1000.f);
-  s.cum_x = n.cum_x - w;
-  s.cum_y = n.cum_y - w * m;
-  s.dist_x = n.dist_x - 2.f * w * m * s.cum_x;
-  s.dist_y = n.dist_y - 2.f * w * s.cum_y;
-  return s;
-}
-
-// safe_div backward, safe-math.slang:68-80.
-__device__ __forceinline__ void safe_div_bwd(float a, float b, float R, float& da, float& db) {
-  da = fabsf(b) < kTiny ? clampf(R / kTiny, kMinVal, kMaxVal) : clampf(R / b, kMinVal, kMaxVal);
-  const float b2 = b * b;
-  db = b2 < kTiny ? clampf(-a / kTiny * R, kMinVal, kMaxVal) : clampf(-a / b2 * R, kMinVal, kMaxVal);
-}
-
-// VJP of update(s, t, dirac) given the cotangent G of the new state. Clamps pass the
-// gradient only strictly inside their range (a zero-density gap gets none).
-__device__ __forceinline__ void update_vjp(const State& s, float t, const State& G, State& Gs, float& Gt,
-                                           float4& Gdirac) {
-  const float dt_raw = t - s.t;
+// One step of the reverse replay: n, the state after the event at t, becomes the state before
+// it, whose own last event was at t_old (inverse_update_dual, spline-machine.slang:65-100),
+// and G, the cotangent of the state after, that of the state before (the VJP of update()).
+// Both share their terms: the weight, the colours and the distance warp are evaluated once.
+// Clamps pass the gradient only strictly inside their range (a zero-density gap gets none);
+// safe_div's backward as safe-math.slang:68-80, its six quotients by two reciprocals (they
+// reach the density and feature gradients only; the colours and the warp, whose terms cancel
+// in the event times' gradients, keep their divisions and powers). The colour sum C is not
+// undone: nothing reads it. Outputs: Gt, Gdirac.
+__device__ __forceinline__ void step_back(State& n, State& G, float t, float4 dirac, float t_old, float& Gt,
+                                          float4& Gdirac) {
+  const float dt_raw = t - t_old;
   const float dt = fmaxf(dt_raw, 0.f);
-  const float area_raw = s.drgb.x * dt;
+  const float4 d = make_float4(n.drgb.x - dirac.x, n.drgb.y - dirac.y, n.drgb.z - dirac.z, n.drgb.w - dirac.w);
+  const float area_raw = d.x * dt;
   const float area = fmaxf(area_raw, 0.f);
-  const float rgb[3] = {safe_div(s.drgb.y, s.drgb.x), safe_div(s.drgb.z, s.drgb.x), safe_div(s.drgb.w, s.drgb.x)};
-  const float ea_in = -area, el_in = -s.logT;
+  const float inv = safe_rcp(d.x);
+  const float dv[3] = {d.y, d.z, d.w};
+  float rgb[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) rgb[i] = safe_div(dv[i], d.x);
+  const float logT = fmaxf(n.logT - area, 0.f);
+  const float ea_in = -area, el_in = -logT;
   const float e1 = safe_exp(ea_in), e2 = safe_exp(el_in);
   const float wraw = (1.f - e1) * e2;
   const float w = clampf(wraw, 0.f, 1.f);
-  const float mid = ((t + s.t) * 0.5f) * 1000.f;
-  const float m = tukey(mid);
-  Gs.dist_x = G.dist_x;
-  Gs.dist_y = G.dist_y;
-  Gs.C = G.C;
-  Gs.drgb = G.drgb;
+  const float mid = ((t + t_old) * 0.5f) * 1000.f;
+  float m, dm;
+  tukey_both(mid, m, dm);
+  const float cum_x = n.cum_x - w, cum_y = n.cum_y - w * m;  // before the event
+
   Gdirac = G.drgb;
-  Gs.logT = 0.f;
-  Gs.t = 0.f;
-  Gt = G.t;
-  float g_area = 0.f;
-  if (area + s.logT > 0.f) {
-    g_area += G.logT;
-    Gs.logT += G.logT;
-  }
+  Gt = 0.f;
+  float Gst = 0.f;
+  float g_area = area + logT > 0.f ? G.logT : 0.f;
+  float GslogT = g_area;
   const float Gc[3] = {G.C.x, G.C.y, G.C.z};
   float g_w = Gc[0] * rgb[0] + Gc[1] * rgb[1] + Gc[2] * rgb[2];
-  g_w += G.dist_x * 2.f * m * s.cum_x + G.dist_y * 2.f * s.cum_y + G.cum_x + G.cum_y * m;
-  const float g_m = G.dist_x * 2.f * w * s.cum_x + G.cum_y * w;
-  Gs.cum_x = G.cum_x + G.dist_x * 2.f * w * m;
-  Gs.cum_y = G.cum_y + G.dist_y * 2.f * w;
-  const float dv[3] = {s.drgb.y, s.drgb.z, s.drgb.w};
+  g_w += G.dist_x * 2.f * m * cum_x + G.dist_y * 2.f * cum_y + G.cum_x + G.cum_y * m;
+  const float g_m = G.dist_x * 2.f * w * cum_x + G.cum_y * w;
+  G.cum_x = G.cum_x + G.dist_x * 2.f * w * m;
+  G.cum_y = G.cum_y + G.dist_y * 2.f * w;
+  const float b2 = d.x * d.x, inv2 = 1.f / (b2 < kTiny ? kTiny : b2);
   float gd[3], gx = 0.f;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    float da, db;
-    safe_div_bwd(dv[i], s.drgb.x, Gc[i] * w, da, db);
-    gd[i] = da;
-    gx += db;
+    const float R = Gc[i] * w;
+    gd[i] = clampf(R * inv, kMinVal, kMaxVal);
+    gx += clampf((-dv[i] * inv2) * R, kMinVal, kMaxVal);
   }
-  Gs.drgb.y += gd[0];
-  Gs.drgb.z += gd[1];
-  Gs.drgb.w += gd[2];
-  Gs.drgb.x += gx;
   if (wraw > 0.f && wraw < 1.f) {
     if (ea_in > kMinVal && ea_in < kLogMax) g_area += g_w * e2 * e1;
-    if (el_in > kMinVal && el_in < kLogMax) Gs.logT += -g_w * (1.f - e1) * e2;
+    if (el_in > kMinVal && el_in < kLogMax) GslogT += -g_w * (1.f - e1) * e2;
   }
   if (area_raw > 0.f) {
-    Gs.drgb.x += g_area * dt;
-    const float g_dt = g_area * s.drgb.x;
+    gx += g_area * dt;
+    const float g_dt = g_area * d.x;
     if (dt_raw > 0.f) {
       Gt += g_dt;
-      Gs.t -= g_dt;
+      Gst -= g_dt;
     }
   }
-  const float g_mid = g_m * dtukey(mid) * 500.f;
+  Gt += G.t;
+  const float g_mid = g_m * dm * 500.f;
   Gt += g_mid;
-  Gs.t += g_mid;
+  Gst += g_mid;
+  G.drgb = make_float4(Gdirac.x + gx, Gdirac.y + gd[0], Gdirac.z + gd[1], Gdirac.w + gd[2]);
+  G.logT = GslogT;
+  G.t = Gst;
+  n.drgb = d;
+  n.t = t_old;
+  n.logT = logT;
+  n.cum_x = cum_x;
+  n.cum_y = cum_y;
 }
 
 __device__ __forceinline__ void inverse4(const float* m, float* inv) {
@@ -467,50 +466,39 @@ __device__ void backward_ray(const BScene& S, const BRayCtx& P, int64_t r, int64
   float acc[kPendingSlots][kGradRow];
 #pragma unroll
   for (int q = 0; q < kPendingSlots; ++q) pj[q] = -1;
-  Ctrl cur = load_ctrl<DEG>(recs, S.features, fstride, ray, B, P.event_log[slot * P.log_cap + (n - 1)]);
+  const int32_t* log = P.event_log + slot * P.log_cap;
+  Ctrl cur = load_ctrl<DEG>(recs, S.features, fstride, ray, B, log[n - 1]);
+  int next = n > 1 ? log[n - 2] : 0;  // the log is read one event ahead of its record
+#pragma unroll 1
   for (int i = n - 1; i >= 0; --i) {
     Ctrl old;
+    old.t = 0.f;
     if (i > 0) {
-      old = load_ctrl<DEG>(recs, S.features, fstride, ray, B, P.event_log[slot * P.log_cap + (i - 1)]);
-    } else {
-      old.t = 0.f;
-      old.dirac = make_float4(0.f, 0.f, 0.f, 0.f);
-      old.j = -1;
+      const int id = next;
+      if (i > 1) next = log[i - 2];
+      old = load_ctrl<DEG>(recs, S.features, fstride, ray, B, id);
     }
-    const State so = inverse_update(s, cur.dirac, old.t);
-    State Gs;
     float Gt;
     float4 Gd;
-    update_vjp(so, cur.t, G, Gs, Gt, Gd);
+    step_back(s, G, cur.t, make_float4(cur.dh, cur.dh * cur.c.x, cur.dh * cur.c.y, cur.dh * cur.c.z), old.t, Gt, Gd);
 
-    const int j = cur.j;
+    const int j = cur.id >> 1;
+    const bool entry = cur.id & 1;
     const Record R = load_record(recs, j);
-    const float sign = cur.entry ? 1.f : -1.f;
+    const float sign = entry ? 1.f : -1.f;
     float gc[3];
     float g_sigma;
     if (DEG == 0) {  // the DC colour: no feature row, no direction gradient
-      const float dh = sign * R.r3.x;
+      const float dh = cur.dh;
       g_sigma = sign * (Gd.x + Gd.y * cur.c.x + Gd.z * cur.c.y + Gd.w * cur.c.z);
       gc[0] = dh * Gd.y;
       gc[1] = dh * Gd.z;
       gc[2] = dh * Gd.w;
     } else {
-      g_sigma = colour_coeffs<DEG>(S, j, sign * R.r3.x, sign, cur.c, Gd, GB, gc);
+      g_sigma = colour_coeffs<DEG>(S, j, cur.dh, sign, cur.c, Gd, GB, gc);
     }
-    // event time: root of |ocn + t rdn|^2 = 1. dt = -(P.docn + t P.drdn) / (P.rdn) with the
-    // hit point in the cancellation-free form P = l +- (sqrt(h)/a) rdn and P.rdn = +-sqrt(h)
-    FullHit H;
-    intersect_full(R, ray, H);
-    const float t = cur.t;
-    const float a_ = fmaf(H.rdn[2], H.rdn[2], fmaf(H.rdn[1], H.rdn[1], H.rdn[0] * H.rdn[0]));
-    const float ba_ = -fmaf(H.ocn[2], H.rdn[2], fmaf(H.ocn[1], H.rdn[1], H.ocn[0] * H.rdn[0])) / a_;
-    const float l_[3] = {fmaf(ba_, H.rdn[0], H.ocn[0]), fmaf(ba_, H.rdn[1], H.ocn[1]), fmaf(ba_, H.rdn[2], H.ocn[2])};
-    const float ll_ = fmaf(l_[2], l_[2], fmaf(l_[1], l_[1], l_[0] * l_[0]));
-    const float sh = sqrtf(fmaxf(a_ * (1.f - ll_), 0.f));
-    const float sg_ = cur.entry ? -1.f : 1.f;
-    const float Pv[3] = {fmaf(sg_ * sh / a_, H.rdn[0], l_[0]), fmaf(sg_ * sh / a_, H.rdn[1], l_[1]),
-                         fmaf(sg_ * sh / a_, H.rdn[2], l_[2])};
-    const float den = sg_ * sh;
+    // event time: root of |ocn + t rdn|^2 = 1. dt = -(P.docn + t P.drdn) / (P.rdn)
+    const float t = cur.t, den = cur.den;
     float gW[9], gmu[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int q = 0; q < 9; ++q) gW[q] = 0.f;
@@ -519,8 +507,8 @@ __device__ void backward_ray(const BScene& S, const BRayCtx& P, int64_t r, int64
       float g_ocn[3], g_rdn[3];
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        g_ocn[a] = k0 * Pv[a];
-        g_rdn[a] = k0 * t * Pv[a];
+        g_ocn[a] = k0 * cur.P[a];
+        g_rdn[a] = k0 * t * cur.P[a];
       }
       const float v[3] = {ray.o.x - R.r0.w, ray.o.y - R.r1.w, ray.o.z - R.r2.w};
       const float dv[3] = {ray.d.x, ray.d.y, ray.d.z};
@@ -562,11 +550,8 @@ __device__ void backward_ray(const BScene& S, const BRayCtx& P, int64_t r, int64
     } else {
       atomicAdd(ag + 3, make_float4(g_sigma, 0.f, 0.f, 0.f));
       const float ev[kGradRow] = {gc[0], gc[1], gc[2]};
-      pending_add<DEG>(S, B, pj, acc, j, cur.entry, ev);
+      pending_add<DEG>(S, B, pj, acc, j, entry, ev);
     }
-    s = so;
-    G = Gs;
-    G.t = Gs.t;
     cur = old;
   }
 
