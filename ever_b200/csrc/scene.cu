@@ -194,9 +194,7 @@ __global__ void k_sort_hist(const uint32_t* __restrict__ keys, int64_t N, int sh
   hist[int64_t(threadIdx.x) * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
-// Exclusive scan of the digit-major histogram in three coalesced kernels: per-chunk
-// sums, a scan of the chunk sums (one block), and a per-chunk scan seeded by it.
-constexpr int kScanChunks = 512;
+constexpr int kScanChunks = 512;  // words after the histogram: digit totals (256 used)
 constexpr int kScanThreads = 256;
 
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* sh, uint32_t& total) {
@@ -226,88 +224,180 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
   return before + x - v;
 }
 
-__global__ void k_scan_sums(const uint32_t* __restrict__ hist, int64_t len, uint32_t* __restrict__ sums) {
-  const int64_t chunk = (len + kScanChunks - 1) / kScanChunks;
-  const int64_t b = blockIdx.x * chunk, e = min(len, b + chunk);
-  uint32_t s = 0;
-  for (int64_t i = b + threadIdx.x; i < e; i += kScanThreads) s += hist[i];
+// Per digit (one block each): exclusive scan of its row of the digit-major histogram, and the
+// row's total.
+__global__ void k_sort_rows(uint32_t* __restrict__ hist, int nblocks, uint32_t* __restrict__ totals) {
   __shared__ uint32_t sh[kScanThreads / 32];
-  uint32_t total;
-  block_exclusive_scan(s, sh, total);
-  if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-__global__ void k_scan_top(uint32_t* __restrict__ sums) {
-  __shared__ uint32_t sh[kScanThreads / 32];
+  uint32_t* row = hist + int64_t(blockIdx.x) * nblocks;
   uint32_t carry = 0;
-  for (int base = 0; base < kScanChunks; base += kScanThreads) {
-    const uint32_t v = sums[base + threadIdx.x];
+  for (int base = 0; base < nblocks; base += kScanThreads) {
+    const int i = base + threadIdx.x;
+    const uint32_t v = i < nblocks ? row[i] : 0u;
     uint32_t total;
     const uint32_t ex = block_exclusive_scan(v, sh, total);
-    sums[base + threadIdx.x] = carry + ex;
+    if (i < nblocks) row[i] = carry + ex;
     carry += total;
   }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
-__global__ void k_scan_chunks(uint32_t* __restrict__ hist, int64_t len, const uint32_t* __restrict__ sums) {
-  const int64_t chunk = (len + kScanChunks - 1) / kScanChunks;
-  const int64_t b = blockIdx.x * chunk, e = min(len, b + chunk);
-  __shared__ uint32_t sh[kScanThreads / 32];
-  uint32_t carry = sums[blockIdx.x];
-  for (int64_t base = b; base < e; base += kScanThreads) {
-    const int64_t i = base + threadIdx.x;
-    const uint32_t v = i < e ? hist[i] : 0u;
-    uint32_t total;
-    const uint32_t ex = block_exclusive_scan(v, sh, total);
-    if (i < e) hist[i] = carry + ex;
-    carry += total;
-  }
+// Rank of this lane's digit among the warp's digits so far: wc is the warp's 256 counters.
+__device__ __forceinline__ uint32_t warp_rank(uint32_t d, uint32_t* wc, uint32_t lt_mask) {
+  const uint32_t peers = __match_any_sync(0xffffffffu, d);
+  const uint32_t before = __popc(peers & lt_mask), at = wc[d];
+  __syncwarp();
+  if (before == 0) wc[d] = at + __popc(peers);
+  __syncwarp();
+  return at + before;
 }
 
-__global__ void k_sort_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                               uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int64_t N, int shift,
-                               const uint32_t* __restrict__ hist, int nblocks) {
-  __shared__ uint32_t gofs[256];
-  __shared__ uint32_t running[256];
+// Stable scatter of one tile: items are ranked warp by warp (a warp's items are contiguous),
+// put in digit order in shared memory and written out in runs of one digit. rows: hist is
+// scanned (k_sort_rows) and totals holds the digit totals; otherwise the block sums the raw
+// rows itself, which for up to kDirectBlocks tiles is cheaper than another launch.
+constexpr int kDirectBlocks = 16;
+__global__ void __launch_bounds__(kSortThreads)
+    k_sort_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
+                   uint32_t* __restrict__ vout, int64_t N, int shift, const uint32_t* __restrict__ hist,
+                   const uint32_t* __restrict__ totals, int nblocks, bool rows) {
   __shared__ uint32_t wcount[kSortWarps][256];
+  __shared__ uint32_t start[256];   // of the digit in the tile
+  __shared__ uint32_t gofs[256];    // output position of the digit's first item, minus start
+  __shared__ uint32_t sk[kSortTile], sv[kSortTile];
+  __shared__ uint32_t sh[kScanThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  gofs[tid] = hist[int64_t(tid) * nblocks + blockIdx.x];
-  running[tid] = 0;
-  for (int w = 0; w < kSortWarps; ++w) wcount[w][tid] = 0;
-  __syncthreads();
-  const int64_t base = int64_t(blockIdx.x) * kSortTile;
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  for (int r = 0; r < kSortItems; ++r) {
-    const int64_t i = base + r * kSortThreads + tid;
-    const bool ok = i < N;
-    uint32_t key = 0, val = 0, d = 256;  // 256: out of range, never matches a real digit
-    if (ok) {
-      key = kin[i];
-      val = vin[i];
-      d = (key >> shift) & 255u;
+  uint32_t before, all;
+  const uint32_t* row = hist + int64_t(tid) * nblocks;
+  if (rows) {
+    before = row[blockIdx.x];
+    all = totals[tid];
+  } else {
+    before = all = 0;
+    for (int b = 0; b < nblocks; ++b) {
+      const uint32_t c = row[b];
+      before += b < int(blockIdx.x) ? c : 0u;
+      all += c;
     }
-    const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    const uint32_t rank_w = __popc(peers & lt_mask);
-    if (ok && rank_w == 0) wcount[warp][d] = __popc(peers);
+  }
+#pragma unroll
+  for (int w = 0; w < kSortWarps; ++w) wcount[w][tid] = 0;
+  const int64_t base = int64_t(blockIdx.x) * kSortTile;
+  const int n = int(min(int64_t(kSortTile), N - base));
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
+#pragma unroll
+  for (int r = 0; r < kSortItems; ++r) {
+    const int i = (warp * kSortItems + r) * 32 + lane;
+    key[r] = i < n ? kin[base + i] : 0xffffffffu;  // past the end: last of the last digit, not written
+    val[r] = i < n ? vin[base + i] : 0u;
+  }
+  uint32_t total;
+  const uint32_t digit0 = block_exclusive_scan(all, sh, total);  // also: the counters are clear
+#pragma unroll
+  for (int r = 0; r < kSortItems; ++r) {
+    const int i = (warp * kSortItems + r) * 32 + lane;
+    rank[r] = warp_rank(i < n ? (key[r] >> shift) & 255u : 255u, wcount[warp], lt_mask);
+  }
+  __syncthreads();
+  uint32_t acc = 0;
+#pragma unroll
+  for (int w = 0; w < kSortWarps; ++w) {
+    const uint32_t c = wcount[w][tid];
+    wcount[w][tid] = acc;
+    acc += c;
+  }
+  const uint32_t st = block_exclusive_scan(acc, sh, total);
+  start[tid] = st;
+  gofs[tid] = digit0 + before - st;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kSortItems; ++r) {
+    const int i = (warp * kSortItems + r) * 32 + lane;
+    const uint32_t d = i < n ? (key[r] >> shift) & 255u : 255u;
+    const uint32_t p = start[d] + wcount[warp][d] + rank[r];
+    sk[p] = key[r];
+    sv[p] = val[r];
+  }
+  __syncthreads();
+  for (int e = tid; e < n; e += kSortThreads) {
+    const uint32_t k = sk[e], dst = gofs[(k >> shift) & 255u] + e;
+    kout[dst] = k;
+    vout[dst] = sv[e];
+  }
+}
+
+// Small sorts: every pass in one block's shared memory, one launch (3 a pass otherwise, each
+// about 2.5 us of latency).
+constexpr int kSmallThreads = 1024, kSmallItems = 8, kSmallSort = kSmallThreads * kSmallItems;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr size_t kSmallSmem = (2 * kSmallSort + kSmallWarps * 256 + 256 + 32) * sizeof(uint32_t);
+__global__ void __launch_bounds__(kSmallThreads)
+    k_sort_small(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, int n, int bits) {
+  extern __shared__ uint32_t sm[];
+  uint32_t* sk = sm;
+  uint32_t* sv = sk + kSmallSort;
+  uint32_t* wcount = sv + kSmallSort;            // [kSmallWarps][256]
+  uint32_t* start = wcount + kSmallWarps * 256;  // [256]
+  uint32_t* sh = start + 256;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  const int per = (n + kSmallThreads - 1) / kSmallThreads;  // items per thread, a warp's contiguous
+  for (int i = tid; i < n; i += kSmallThreads) {
+    sk[i] = keys[i];
+    sv[i] = vals[i];
+  }
+  for (int shift = 0; shift < bits; shift += 8) {
+    for (int i = tid; i < kSmallWarps * 256; i += kSmallThreads) wcount[i] = 0;
     __syncthreads();
-    {
-      uint32_t acc = running[tid];
-      for (int w = 0; w < kSortWarps; ++w) {
-        const uint32_t c = wcount[w][tid];
-        wcount[w][tid] = acc;
+    uint32_t key[kSmallItems], val[kSmallItems], rank[kSmallItems];
+#pragma unroll
+    for (int r = 0; r < kSmallItems; ++r) {
+      if (r >= per) break;
+      const int i = (warp * per + r) * 32 + lane;
+      key[r] = i < n ? sk[i] : 0xffffffffu;
+      val[r] = i < n ? sv[i] : 0u;
+      rank[r] = warp_rank(i < n ? (key[r] >> shift) & 255u : 255u, wcount + warp * 256, lt_mask);
+    }
+    __syncthreads();
+    uint32_t acc = 0;
+    if (tid < 256) {
+#pragma unroll 8
+      for (int w = 0; w < kSmallWarps; ++w) {
+        const uint32_t c = wcount[w * 256 + tid];
+        wcount[w * 256 + tid] = acc;
         acc += c;
       }
-      running[tid] = acc;
+    }
+    uint32_t x = acc;  // inclusive scan over the 256 digits (8 warps)
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (tid < 256 && lane == 31) sh[warp] = x;
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t before = 0;
+      for (int w = 0; w < warp; ++w) before += sh[w];
+      start[tid] = before + x - acc;
     }
     __syncthreads();
-    if (ok) {
-      const uint32_t dst = gofs[d] + wcount[warp][d] + rank_w;
-      kout[dst] = key;
-      vout[dst] = val;
+#pragma unroll
+    for (int r = 0; r < kSmallItems; ++r) {
+      if (r >= per) break;
+      const int i = (warp * per + r) * 32 + lane;
+      if (i < n) {
+        const uint32_t d = (key[r] >> shift) & 255u;
+        const uint32_t p = start[d] + wcount[warp * 256 + d] + rank[r];
+        sk[p] = key[r];
+        sv[p] = val[r];
+      }
     }
     __syncthreads();
-    for (int w = 0; w < kSortWarps; ++w) wcount[w][tid] = 0;
-    __syncthreads();
+  }
+  for (int i = tid; i < n; i += kSmallThreads) {
+    keys[i] = sk[i];
+    vals[i] = sv[i];
   }
 }
 
@@ -497,15 +587,21 @@ int sort_blocks(int64_t N) { return int(div_up(std::max<int64_t>(N, 1), kSortTil
 // hist holds sort_blocks(N) * 256 words.
 void sort_pairs(uint32_t*& ka, uint32_t*& va, uint32_t*& kb, uint32_t*& vb, uint32_t* hist, int64_t N, int bits,
                 cudaStream_t st) {
+  if (N <= kSmallSort) {
+    if (cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmallSmem)) ==
+        cudaSuccess) {
+      k_sort_small<<<1, kSmallThreads, kSmallSmem, st>>>(ka, va, int(N), bits);
+      return;
+    }
+    cudaGetLastError();  // the general path needs no opt-in
+  }
   const int nblocks = sort_blocks(N);
-  const int64_t len = int64_t(nblocks) * 256;
-  uint32_t* sums = hist + len;  // kScanChunks words after the histogram
+  uint32_t* totals = hist + int64_t(nblocks) * 256;  // within the kScanChunks words after the histogram
+  const bool rows = nblocks > kDirectBlocks;
   for (int shift = 0; shift < bits; shift += 8) {
     k_sort_hist<<<nblocks, kSortThreads, 0, st>>>(ka, N, shift, hist, nblocks);
-    k_scan_sums<<<kScanChunks, kScanThreads, 0, st>>>(hist, len, sums);
-    k_scan_top<<<1, kScanThreads, 0, st>>>(sums);
-    k_scan_chunks<<<kScanChunks, kScanThreads, 0, st>>>(hist, len, sums);
-    k_sort_scatter<<<nblocks, kSortThreads, 0, st>>>(ka, va, kb, vb, N, shift, hist, nblocks);
+    if (rows) k_sort_rows<<<256, kScanThreads, 0, st>>>(hist, nblocks, totals);
+    k_sort_scatter<<<nblocks, kSortThreads, 0, st>>>(ka, va, kb, vb, N, shift, hist, totals, nblocks, rows);
     std::swap(ka, kb);
     std::swap(va, vb);
   }
