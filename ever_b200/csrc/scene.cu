@@ -485,59 +485,54 @@ __global__ void k_lbvh(const uint32_t* __restrict__ codes, int64_t N, Node* __re
   } while (t > 1);
   const int64_t gamma = i + s * d + min(d, 0);
   const int64_t lo = min(i, j), hi = max(i, j);
+  const int up = int(i) << 1;  // parent link: 2 * node + which half (N < 2^30)
   int c0, c1;
   if (lo == gamma) {
     c0 = ~int(gamma);
-    parent_leaf[gamma] = int(i);
+    parent_leaf[gamma] = up;
   } else {
     c0 = int(gamma);
-    parent_node[gamma] = int(i);
+    parent_node[gamma] = up;
   }
   if (hi == gamma + 1) {
     c1 = ~int(gamma + 1);
-    parent_leaf[gamma + 1] = int(i);
+    parent_leaf[gamma + 1] = up | 1;
   } else {
     c1 = int(gamma + 1);
-    parent_node[gamma + 1] = int(i);
+    parent_node[gamma + 1] = up | 1;
   }
   nodes[i].b.z = __int_as_float(c0);
   nodes[i].d.z = __int_as_float(c1);
   if (i == 0) parent_node[0] = -1;
 }
 
-__device__ __forceinline__ void child_box(const Node* nodes, const float4* aabb, int c, float3& lo, float3& hi) {
-  if (c < 0) {
-    const float4 a = __ldcg(aabb + 2 * int64_t(~c)), b = __ldcg(aabb + 2 * int64_t(~c) + 1);
-    lo = make_float3(a.x, a.y, a.z);
-    hi = make_float3(b.x, b.y, b.z);
-  } else {
-    const float4 a = __ldcg(&nodes[c].a), b = __ldcg(&nodes[c].b), cc = __ldcg(&nodes[c].c), d = __ldcg(&nodes[c].d);
-    lo = make_float3(fminf(a.x, cc.x), fminf(a.y, cc.y), fminf(a.z, cc.z));
-    hi = make_float3(fmaxf(a.w, cc.w), fmaxf(b.x, d.x), fmaxf(b.y, d.y));
-  }
-}
-
+// Bottom-up refit, one thread per leaf: it stores the box it carries in its half of the parent
+// and goes on only as the second to arrive, with the box of both halves. A level costs two
+// round trips to L2, the atomic and the sibling's half (which its thread stored before its
+// own atomic); reading links and children's nodes instead took four (1M ellipsoids 141 us,
+// 1,000 24 us).
 __global__ void k_refit(int64_t N, Node* __restrict__ nodes, const float4* __restrict__ aabb,
                         const int32_t* __restrict__ parent_node, const int32_t* __restrict__ parent_leaf,
                         uint32_t* __restrict__ flags) {
   const int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (j >= N) return;
-  int n = parent_leaf[j];
-  while (n >= 0) {
-    // acquire-release at device scope: this thread's box stores above happen before the
-    // sibling's loads once it sees the count, and the sibling's stores before this thread's
-    // loads below (one instruction instead of two full fences around the atomic)
+  float4 lo = aabb[2 * j], hi = aabb[2 * j + 1];
+  int up = parent_leaf[j];
+  while (up >= 0) {
+    const int n = up >> 1;
+    float4* own = reinterpret_cast<float4*>(nodes + n) + 2 * (up & 1);
+    const float4* other = reinterpret_cast<const float4*>(nodes + n) + 2 * (1 - (up & 1));
+    up = __ldg(parent_node + n);
+    __stcg(own, make_float4(lo.x, lo.y, lo.z, hi.x));
+    __stcg(reinterpret_cast<float2*>(own + 1), make_float2(hi.y, hi.z));  // the link stays
+    // acquire-release at device scope: this thread's stores above happen before the sibling's
+    // loads once it sees the count, and the sibling's stores before this thread's loads below
+    // (one instruction instead of two full fences around the atomic)
     cuda::atomic_ref<uint32_t, cuda::thread_scope_device> f(flags[n]);
     if (f.fetch_add(1u, cuda::memory_order_acq_rel) == 0u) return;  // the sibling subtree is not done yet
-    const float c0 = __ldcg(&nodes[n].b.z), c1 = __ldcg(&nodes[n].d.z);
-    float3 l0, h0, l1, h1;
-    child_box(nodes, aabb, __float_as_int(c0), l0, h0);
-    child_box(nodes, aabb, __float_as_int(c1), l1, h1);
-    __stcg(&nodes[n].a, make_float4(l0.x, l0.y, l0.z, h0.x));
-    __stcg(&nodes[n].b, make_float4(h0.y, h0.z, c0, 0.f));
-    __stcg(&nodes[n].c, make_float4(l1.x, l1.y, l1.z, h1.x));
-    __stcg(&nodes[n].d, make_float4(h1.y, h1.z, c1, 0.f));
-    n = parent_node[n];
+    const float4 a = __ldcg(other), b = __ldcg(other + 1);
+    lo = make_float4(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z), 0.f);
+    hi = make_float4(fmaxf(hi.x, a.w), fmaxf(hi.y, b.x), fmaxf(hi.z, b.y), 0.f);
   }
 }
 
