@@ -401,12 +401,13 @@ __global__ void __launch_bounds__(kSmallThreads)
   }
 }
 
-// Gathers records, features and leaf boxes into Morton order.
+// Gathers records and leaf boxes into Morton order. dc_feat: the feature rows of a scene that
+// keeps only each record's DC colour (null: not written here).
 __global__ void k_gather(const uint32_t* __restrict__ sorted_vals, int64_t N, int K,
                          const float* __restrict__ mean, const float* __restrict__ scale,
                          const float* __restrict__ quat, const float* __restrict__ density,
                          const float4* __restrict__ aabb_in,
-                         float4* __restrict__ aabb_out, Record* __restrict__ recs, float* __restrict__ feat_out,
+                         float4* __restrict__ aabb_out, Record* __restrict__ recs, const float* __restrict__ dc_feat,
                          int32_t* __restrict__ order) {
   const int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (j >= N) return;
@@ -419,12 +420,18 @@ __global__ void k_gather(const uint32_t* __restrict__ sorted_vals, int64_t N, in
   R.r0 = make_float4(W[0], W[1], W[2], mu.x);
   R.r1 = make_float4(W[3], W[4], W[5], mu.y);
   R.r2 = make_float4(W[6], W[7], W[8], mu.z);
-  // r3.yzw (the DC colour) is written by k_gather_features, and kept by a refit without features
+  // r3.yzw (the DC colour) is written here from dc_feat, or by k_gather_features, or kept by a
+  // refit without features
   float4* rp = reinterpret_cast<float4*>(recs + j);
   rp[0] = R.r0;
   rp[1] = R.r1;
   rp[2] = R.r2;
-  recs[j].r3.x = density[p];
+  if (dc_feat) {
+    const float* f = dc_feat + p * (3 * K);
+    rp[3] = make_float4(density[p], dc_channel(__ldg(f)), dc_channel(__ldg(f + 1)), dc_channel(__ldg(f + 2)));
+  } else {
+    recs[j].r3.x = density[p];
+  }
   aabb_out[2 * j] = aabb_in[2 * p];
   aabb_out[2 * j + 1] = aabb_in[2 * p + 1];
 }
@@ -661,8 +668,8 @@ cudaError_t scene_build(const float* mean, const float* scale, const float* quat
   // 30-bit keys: 4 passes of 8 bits
   sort_pairs(ka, va, kb, vb, hist, N, 30, st);
   k_gather<<<unsigned(gb), tb, 0, st>>>(va, N, K, mean, scale, quat, density, aabb_a, aabb_b,
-                                        reinterpret_cast<Record*>(sc->records), sc->features, sc->order);
-  launch_gather_features(sc->order, N, K, feat, sc->features, sc->records, st);
+                                        reinterpret_cast<Record*>(sc->records), dc_only ? feat : nullptr, sc->order);
+  if (!dc_only) launch_gather_features(sc->order, N, K, feat, sc->features, sc->records, st);
   if (N == 1) {
     k_single_leaf<<<1, 1, 0, st>>>(nodes, aabb_b);
     return cudaGetLastError();
@@ -693,9 +700,9 @@ cudaError_t scene_refit(const float* mean, const float* scale, const float* quat
   const int64_t gb = div_up(N, tb);
   k_aabbs<<<unsigned(gb), tb, 0, st>>>(mean, scale, quat, N, aabb_a, bounds);
   k_gather<<<unsigned(gb), tb, 0, st>>>(reinterpret_cast<const uint32_t*>(sc->order), N, K, mean, scale, quat, density,
-                                        aabb_a, aabb_b, reinterpret_cast<Record*>(sc->records), sc->features,
-                                        sc->order);
-  if (feat)
+                                        aabb_a, aabb_b, reinterpret_cast<Record*>(sc->records),
+                                        sc->features ? nullptr : feat, sc->order);
+  if (feat && sc->features)
     launch_gather_features(sc->order, N, K, feat, sc->features, sc->records, st);
   if (N == 1) {
     k_single_leaf<<<1, 1, 0, st>>>(nodes, aabb_b);
