@@ -25,6 +25,7 @@ from torch.autograd import Function
 
 from . import _native as N
 from . import tracer as T
+from .tracer import _stream, on_device
 
 
 @dataclass
@@ -67,10 +68,6 @@ def _device(device):
     return torch.device(device) if device is not None else torch.device("cuda", torch.cuda.current_device())
 
 
-def _stream(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
-
-
 def _jitter(jitter, R, device):
     if jitter is None:
         return None
@@ -90,7 +87,7 @@ def camera_rays(width, height, fx, fy, c2w, cx=None, cy=None, jitter=None, devic
     rayo = torch.empty((R, 3), dtype=torch.float32, device=device)
     rayd = torch.empty((R, 3), dtype=torch.float32, device=device)
     jitter = _jitter(jitter, R, device)
-    with torch.cuda.device(device):
+    with on_device(device):
         N.check(N.load().ever_camera_rays(ctypes.byref(cam), N.ptr(jitter), N.ptr(rayo), N.ptr(rayd),
                                           _stream(device)))
     return rayo, rayd
@@ -118,7 +115,7 @@ def slot_pixels(camera: Camera, device=None) -> torch.Tensor:
     """(slots,) int32: the pixel each slot of a camera trace traces, -1 for padding."""
     device = _device(device)
     out = torch.empty(camera_slots(camera), dtype=torch.int32, device=device)
-    with torch.cuda.device(device):
+    with on_device(device):
         N.check(N.load().ever_camera_slot_pixels(ctypes.byref(camera.c()), N.ptr(out), _stream(device)))
     return out
 
@@ -151,7 +148,7 @@ def forward(scene: T.Scene, camera: Camera, jitter=None, tmin=0.0, tmax=1000.0, 
     args = T.trace_args(tmin, tmax, max_iters, sh_degree)
     tune = tune or T.Tune()
     lib = N.load()
-    with torch.cuda.device(device):
+    with on_device(device):
         if regrouped and tune.kbuf <= 16:
             ws = torch.empty(max(int(lib.ever_trace_forward_workspace_bytes(S)), 256), dtype=torch.uint8,
                              device=device)
@@ -174,7 +171,7 @@ def backward_order(camera: Camera, fwd: T.ForwardResult, shift: int = 0) -> torc
     need = int(lib.ever_ray_order_workspace_bytes(S))
     ws = torch.empty(max(need, 256), dtype=torch.uint8, device=device)
     order = torch.empty(S, dtype=torch.int32, device=device)
-    with torch.cuda.device(device):
+    with on_device(device):
         N.check(lib.ever_camera_backward_slot_order(ctypes.byref(camera.c()), N.ptr(fwd.iters), int(shift),
                                                     N.ptr(ws), int(ws.numel()), N.ptr(order), _stream(device)))
     return order
@@ -211,7 +208,7 @@ def backward(scene: T.Scene, camera: Camera, fwd: T.ForwardResult, grad_out, jit
     o.dmean, o.dscale, o.dquat, o.ddensity = N.ptr(g.mean), N.ptr(g.scale), N.ptr(g.quat), N.ptr(g.density)
     o.dfeatures, o.drayo, o.drayd, o.dmeans2d = N.ptr(g.features), N.ptr(g.rayo), N.ptr(g.rayd), N.ptr(g.means2d)
     args = T.trace_args(tmin, tmax, max_iters, sh_degree)
-    with torch.cuda.device(device):
+    with on_device(device):
         N.check(lib.ever_trace_backward_camera(
             ctypes.byref(scene.c), ctypes.byref(camera.c()), N.ptr(jitter), ctypes.byref(args), N.ptr(grad_out),
             N.ptr(fwd.states), N.ptr(fwd.iters), N.ptr(fwd.event_log), fwd.event_log.shape[1], N.ptr(wct), num_wct,
@@ -227,7 +224,7 @@ def tri_collection(scene: T.Scene, camera: Camera, fwd: T.ForwardResult, max_ite
     if log is None or R == 0 or max_iters <= 0:
         return torch.zeros(R * max(int(max_iters), 0), dtype=torch.int32, device=scene.device)
     tri = torch.empty(R * int(max_iters), dtype=torch.int32, device=scene.device)
-    with torch.cuda.device(scene.device):
+    with on_device(scene.device):
         N.check(N.load().ever_camera_event_log_to_reference(ctypes.byref(scene.c), ctypes.byref(camera.c()),
                                                             N.ptr(log), log.shape[1], N.ptr(fwd.iters), N.ptr(tri),
                                                             int(max_iters), _stream(scene.device)))

@@ -11,17 +11,13 @@ as (N,1,3), computed in one kernel (and one backward kernel) instead of three pa
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Any
 
 import torch
 from torch.autograd import Function
 
 from . import _native as N
-
-
-def _stream(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+from .tracer import _stream, on_device
 
 
 def _check(means, features, cam, sh_degree):
@@ -41,7 +37,7 @@ def _check(means, features, cam, sh_degree):
 def _run(means, features, cam, sh_degree, mode, grad_out=None):
     lib = N.load()
     n, k = means.shape[0], features.shape[1]
-    with torch.cuda.device(means.device):
+    with on_device(means.device):
         if grad_out is None:
             out = torch.empty((n, 3), dtype=torch.float32, device=means.device)
             N.check(lib.ever_sh_prepass(N.ptr(means), N.ptr(features), n, k, int(sh_degree), N.ptr(cam), mode,

@@ -44,6 +44,9 @@ from torch.autograd import Function
 from . import tracer as T
 
 _SIDE_STREAMS: dict = {}
+# Up to these sizes the call is bound by its host side, and the events and the stream switch of
+# an overlapped ray order cost more (about 30 us) than the order does on the GPU.
+_SMALL_RAYS, _SMALL_PRIMS = 32768, 65536
 
 
 def _side_stream(device) -> torch.cuda.Stream:
@@ -101,7 +104,11 @@ class SplineTracer(Function):
                     ray_order = None
         if isinstance(ray_order, str) and ray_order != "auto":
             raise RuntimeError(f"ray_order must be 'auto', None or an int32 tensor, got {ray_order!r}")
-        if isinstance(ray_order, str) and rayo.shape[0] > 0 and rayo.is_cuda:
+        small = rayo.shape[0] <= _SMALL_RAYS and mean.shape[0] <= _SMALL_PRIMS
+        if isinstance(ray_order, str) and rayo.shape[0] > 0 and rayo.is_cuda and small:
+            ray_order = T.ray_order(rayo, rayd)
+            scene = T.Scene(mean, scale, quat, density, color, dc_only=not sh_degree)
+        elif isinstance(ray_order, str) and rayo.shape[0] > 0 and rayo.is_cuda:
             # the coherent ray order needs only the rays: it runs on a side stream while the
             # BVH is built on the caller's stream
             main = torch.cuda.current_stream(rayo.device)

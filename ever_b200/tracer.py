@@ -5,6 +5,7 @@ libever_b200.so. Nothing here synchronises the host.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from dataclasses import dataclass
 from typing import Optional
@@ -28,8 +29,23 @@ def _check_tensor(name, t, device, last_dim=None, dtype=torch.float32):
         raise RuntimeError(f"{name} must have last dimension with size {last_dim}")
 
 
+# The host side of a small trace is as long as its kernels (about 5 us for each device guard
+# and stream object of torch.cuda), so the current stream is read as a plain handle and the
+# device is switched only when it is not the current one.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_no_switch = contextlib.nullcontext()
+
+
 def _stream(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    if _raw_stream is None:
+        return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return ctypes.c_void_p(_raw_stream(index))
+
+
+def on_device(device):
+    """torch.cuda.device(device), for nothing when it is the current device already."""
+    return _no_switch if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 @dataclass
@@ -81,7 +97,7 @@ class Scene:
         self.workspace = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
         self.c = N.EverScene()
         m, s, q, d, f = self.tensors
-        with torch.cuda.device(device):
+        with on_device(device):
             build = lib.ever_scene_build_dc if self.dc_only else lib.ever_scene_build
             N.check(build(N.ptr(m), N.ptr(s), N.ptr(q), N.ptr(d), N.ptr(f), n, self.sh_coeffs,
                           N.ptr(self.workspace), int(self.workspace.numel()), ctypes.byref(self.c), _stream(device)))
@@ -93,7 +109,7 @@ class Scene:
         recorded in a CUDA graph keep working across rebuilds.
         """
         m, s, q, d, f = self.tensors
-        with torch.cuda.device(self.device):
+        with on_device(self.device):
             lib = N.load()
             build = lib.ever_scene_build_dc if self.dc_only else lib.ever_scene_build
             N.check(build(N.ptr(m), N.ptr(s), N.ptr(q), N.ptr(d), N.ptr(f), self.num_prims, self.sh_coeffs,
@@ -104,7 +120,7 @@ class Scene:
         """Refits the BVH in place to the (updated) input tensors, keeping the last build's
         Morton order and tree topology: cheaper than rebuild() between small updates."""
         m, s, q, d, f = self.tensors
-        with torch.cuda.device(self.device):
+        with on_device(self.device):
             N.check(N.load().ever_scene_refit(N.ptr(m), N.ptr(s), N.ptr(q), N.ptr(d),
                                               N.ptr(f) if with_features else None, N.ptr(self.workspace),
                                               int(self.workspace.numel()), ctypes.byref(self.c),
@@ -116,7 +132,7 @@ class Scene:
             raise RuntimeError("All inputs (colors) must have the same 0 dimension")
         f = features.contiguous()
         self.tensors = self.tensors[:4] + (f,)
-        with torch.cuda.device(self.device):
+        with on_device(self.device):
             N.check(N.load().ever_scene_set_features(ctypes.byref(self.c), N.ptr(f), _stream(self.device)))
 
 
@@ -187,7 +203,7 @@ def forward(scene: Scene, rayo, rayd, tmin=0.0, tmax=1000.0, max_iters=500, sh_d
     args = trace_args(tmin, tmax, max_iters, sh_degree, depth_hint)
     tune = tune or Tune()
     lib = N.load()
-    with torch.cuda.device(device):
+    with on_device(device):
         # the packed passes pay for buffers of up to 16 events; with 32, most rays finish in
         # the first round and the extra passes only add their overhead
         if regrouped and tune.traversal in (0, 2) and tune.kbuf <= 16 and R < (1 << 31):
@@ -250,7 +266,7 @@ def backward(scene: Scene, rayo, rayd, fwd: ForwardResult, grad_out, tmin=0.0, t
     common = (ctypes.byref(scene.c), N.ptr(rayo), N.ptr(rayd), R, ctypes.byref(args), N.ptr(grad_out),
               N.ptr(fwd.states), N.ptr(fwd.iters), N.ptr(fwd.event_log), fwd.event_log.shape[1], N.ptr(wct), num_wct,
               N.ptr(m), N.ptr(s), N.ptr(q), N.ptr(workspace), int(workspace.numel()), N.ptr(ray_order))
-    with torch.cuda.device(device):
+    with on_device(device):
         if slot_order is None:
             N.check(lib.ever_trace_backward(*common, ctypes.byref((tune or Tune()).c()), ctypes.byref(o),
                                             _stream(device)))
@@ -272,7 +288,7 @@ def backward_order(fwd: ForwardResult, ray_order=None, shift: int = 1,
     need = int(lib.ever_ray_order_workspace_bytes(R))
     if workspace is None or workspace.numel() < need:
         workspace = torch.empty(max(need, 256), dtype=torch.uint8, device=device)
-    with torch.cuda.device(device):
+    with on_device(device):
         N.check(lib.ever_backward_slot_order(N.ptr(fwd.iters), N.ptr(ray_order), R, int(shift), N.ptr(workspace),
                                              int(workspace.numel()), N.ptr(order), _stream(device)))
     return order
@@ -291,7 +307,7 @@ def ray_order(rayo, rayd, workspace: torch.Tensor | None = None) -> torch.Tensor
     need = int(lib.ever_ray_order_workspace_bytes(R))
     if workspace is None or workspace.numel() < need:
         workspace = torch.empty(max(need, 256), dtype=torch.uint8, device=device)
-    with torch.cuda.device(device):
+    with on_device(device):
         N.check(lib.ever_ray_order(N.ptr(rayo), N.ptr(rayd), R, N.ptr(workspace), int(workspace.numel()),
                                    N.ptr(order), _stream(device)))
     return order
@@ -304,7 +320,7 @@ def reference_tri_collection(scene: Scene, fwd: ForwardResult, max_iters: int, r
     if log is None or R == 0 or max_iters <= 0:
         return torch.zeros(R * max(int(max_iters), 0), dtype=torch.int32, device=scene.device)
     tri = torch.empty(R * int(max_iters), dtype=torch.int32, device=scene.device)
-    with torch.cuda.device(scene.device):
+    with on_device(scene.device):
         N.check(N.load().ever_event_log_to_reference(ctypes.byref(scene.c), N.ptr(log),
                                                      0 if log is None else log.shape[1], N.ptr(fwd.iters), R,
                                                      N.ptr(ray_order), N.ptr(tri), int(max_iters),
