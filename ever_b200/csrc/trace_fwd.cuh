@@ -550,16 +550,19 @@ __device__ __forceinline__ bool run_rounds(const SceneRef& sc, const TraceCtx& C
 // leaves of the whole t range do not fit, the phase goes on in stages over t. At 1M
 // ellipsoids / 1080p the forward's kernels took 6.26 ms before (one walk over whole nodes,
 // no cone test, integration where an event became final, a second pass of stack rounds for
-// overflowing packets) and take 3.6 ms; a packet issues 34k instructions, 66k before.
+// overflowing packets) and take 3.5 ms; a packet issues 33k instructions, 66k before.
 // Rays in no order (no_order) have no list in common and go to the rounds at once.
-// Events a lane holds in the frustum phase. More only cost registers: at 1M ellipsoids /
-// 1080p a lane holds more than 5 on 3% of the leaves, and a lane that runs out makes another
-// pass over the list (8: 3.6 ms, 12: 4.1 ms).
-constexpr int frustum_buffer(int kbuf) { return kbuf == 32 ? 16 : 8; }
-constexpr int kLowEvents = 2;      // buffered events up to which an insertion moves only the first entries
-constexpr int kHold = 4;           // leaves between two rounds of ordering
-constexpr int kWalkCap = 256;      // nodes waiting in the walk
-constexpr int kFirstLeaves = 128;  // leaves of a group's first stage
+// Events a lane holds in the frustum phase: more cost registers and compares, fewer cost the
+// lanes that run out another pass over the list (kernel time at 1M ellipsoids / 1080p and for
+// 100,000 dense ones at 800 x 800 with 8 / 10 / 12 / 16 events: 3.58 / 3.49 / 3.56 / 3.83 and
+// 1.68 / 1.57 / 1.48 / 1.49 ms).
+constexpr int frustum_buffer(int kbuf) { return kbuf == 32 ? 16 : (kbuf == 8 ? 8 : 10); }
+constexpr int kLowEvents = 4;  // buffered events up to which an insertion moves only the first entries
+constexpr int kHold = 4;       // leaves between two rounds of ordering (2: 3.59, 8: 3.51 ms)
+constexpr int kWalkCap = 256;  // nodes waiting in the walk
+// Leaves of a group's first stage. Fewer prune the walk sooner, but a group that needs more
+// walks again: 96: 3.68 ms (dense 2.98), 192: 3.49 (2M ellipsoids 3.75 against 3.59 with 128).
+constexpr int kFirstLeaves = 128;
 constexpr int kStageLeaves = 256;  // leaves of a later stage
 constexpr int kCandCap = kStageLeaves + 64;
 constexpr int kMaxCuts = 6;      // of a list that overflows in one walk
@@ -972,9 +975,8 @@ __device__ __forceinline__ void sort_keys(uint64_t* cand, int n, int lane) {
 static_assert(kStageLeaves <= 256, "sort_keys takes up to 256 keys");
 
 // The sorted leaf list of a group of the warp's rays (the lanes with `mine`) within [t_lo,
-// cap]: bounds, walk and sort, over the warp's lists at smem[at]. A call of its own: the walk
-// and the passes over its list then keep their registers apart (in one piece, small changes
-// moved the kernel by 10%). Returns the number of leaves (packet_leaves) and the cap.
+// cap]: bounds, walk and sort, over the warp's lists at smem[at]. A call of its own, so that
+// the walk and the passes over its list keep their registers apart. Returns the number of leaves (packet_leaves) and the cap.
 struct LeafList {
   int n;
   float cap;
@@ -1128,10 +1130,7 @@ __device__ __forceinline__ void order_events(const SceneRef& sc, const TraceCtx&
         }
         if (C.out.touch_count) atomicAdd(C.out.touch_count + __ldg(sc.order + j), 1);
         ++L.iters;
-        if (++L.cnt16 == kRefRound) {
-          L.s16 = t;
-          L.cnt16 = 0;
-        }
+        if ((L.iters & (kRefRound - 1)) == 0) L.s16 = t;
         done = !(depth < kLogCutoff && L.iters < C.max_iters);
       }
       if (done) live = act = false;
@@ -1324,6 +1323,7 @@ __device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx
       grp = half_group(grp, lane);
     }
   }
+  L.cnt16 = L.iters & (kRefRound - 1);
   L.s = ring_state_load(q.st, lane);
   if (L.iters > first) L.last_dirac = event_dirac<DEG>(sc, B, bs, __float_as_uint(q.st[32 * 13 + lane]));
   __syncwarp();
@@ -1409,7 +1409,7 @@ __device__ __forceinline__ RayLoop resume_ray(const EverForwardOut& out, int64_t
 
 // Resident blocks per SM that the register budget of the packet kernels targets: 16 warps
 // (128 registers) with the frustum phase, which is bound by instructions and not by latency
-// (3.6 ms at 1M ellipsoids / 1080p; 20 warps: 3.8, 24: 3.9 ms, with spills); 20 warps (96
+// (3.6 ms at 1M ellipsoids / 1080p; 20 warps: 4.0 ms, with spills); 20 warps (96
 // registers) for the rounds, whose traversal is latency-bound.
 template <int BLOCK, bool FRUSTUM = true>
 struct FwdMinBlocks {
