@@ -765,6 +765,8 @@ __global__ void k_finalize(const FinalizeParams P) {
   }
   for (int i = 0; i < 4; ++i) P.out.dquat[4 * p + i] = clip_grad(gq[i], 1e3f);
   P.out.ddensity[p] = clip_grad(g[12], 50.f);
+  if (P.dc_only && P.K == 1)
+    for (int i = 0; i < 3; ++i) P.out.dfeatures[3 * p + i] = clip_grad(g[13 + i], 1e3f);
 
   if (single_wct) {
     const float mx = P.mean[3 * p], my = P.mean[3 * p + 1], mz = P.mean[3 * p + 2];
@@ -778,7 +780,9 @@ __global__ void k_finalize(const FinalizeParams P) {
 // threadIdx.y, one float4 column per threadIdx.x (blockDim.x = feat_stride(K) / 4). vec: the
 // output rows are whole, 16-byte aligned float4s (3K % 4 == 0, aligned base). The DC
 // gradient of degree-0 traces sits in the pad floats 13..15 of the geometry row and is
-// added to coefficient 0; dc_only: the feature rows were not used (all zero, not read).
+// added to coefficient 0; dc_only: the feature rows were not used (all zero, not read). With
+// K = 1 the row is that gradient and k_finalize writes it, so this kernel is not launched;
+// with K > 1 writing three floats a row there and clearing the rest took as long as it does.
 __global__ void k_finalize_features(const int32_t* __restrict__ order, int64_t N, int K,
                                     const float* __restrict__ acc_feat, const float* __restrict__ acc_geo,
                                     bool dc_only, float* __restrict__ dfeat, bool vec) {
@@ -935,6 +939,7 @@ cudaError_t launch_finalize(const FinalizeParams& P, cudaStream_t st) {
   if (P.N == 0) return cudaSuccess;
   k_inverse_order<<<unsigned((P.N + 255) / 256), 256, 0, st>>>(P.order, P.N, P.inv_order);
   k_finalize<<<unsigned((P.N + 255) / 256), 256, 0, st>>>(P);
+  if (P.dc_only && P.K == 1) return cudaGetLastError();
   const int cols = feat_stride(P.K) / 4, rows = 256 / cols > 0 ? 256 / cols : 1;
   const bool vec = (3 * P.K) % 4 == 0 && reinterpret_cast<uintptr_t>(P.out.dfeatures) % 16 == 0;
   k_finalize_features<<<unsigned((P.N + rows - 1) / rows), dim3(cols, rows), 0, st>>>(
