@@ -558,14 +558,19 @@ __device__ __forceinline__ bool run_rounds(const SceneRef& sc, const TraceCtx& C
 // 1.68 / 1.57 / 1.48 / 1.49 ms).
 constexpr int frustum_buffer(int kbuf) { return kbuf == 32 ? 16 : (kbuf == 8 ? 8 : 10); }
 constexpr int kLowEvents = 4;  // buffered events up to which an insertion moves only the first entries
-constexpr int kHold = 4;       // leaves between two rounds of ordering (2: 3.59, 8: 3.51 ms)
+constexpr int kHold = 4;       // leaves between two rounds of ordering (8: 3.51 ms)
 constexpr int kWalkCap = 256;  // nodes waiting in the walk
 // Leaves of a group's first stage. Fewer prune the walk sooner, but a group that needs more
-// walks again: 96: 3.68 ms (dense 2.98), 192: 3.49 (2M ellipsoids 3.75 against 3.59 with 128).
+// walks again. With 96: 3.68 against 3.60 ms then (dense 2.98 against 1.69); with 192: 3.49
+// against 3.49 (2M ellipsoids 3.75 against 3.59).
 constexpr int kFirstLeaves = 128;
 constexpr int kStageLeaves = 256;  // leaves of a later stage
 constexpr int kCandCap = kStageLeaves + 64;
-constexpr int kMaxCuts = 6;      // of a list that overflows in one walk
+// Cuts of a list that overflows in one walk, for packets with a cone (6 without one: such a
+// group is better traced by the rounds). With 6 for all, packets through dense ellipsoids gave
+// up and were halved again and again: one took 3.3 ms where all 20,000 take 1.6 ms. With 64 the
+// wide packets of small views cut too long (batched views 4.4 -> 5.0 ms).
+constexpr int kMaxCuts = 16;
 constexpr int kMaxStages = 128;  // then the rounds take over
 constexpr int kTileWords = 24;
 constexpr int kStateWords = 14;  // of a lane's integration state: State (13), the last event's id
@@ -914,7 +919,8 @@ __device__ __forceinline__ int packet_leaves(const Node* __restrict__ nodes, con
       if (cull) nc = checked = cull_leaves(tile, recs, cand, checked, nc, lane);
       if (nc > limit) {
         nc = checked = nearer_leaves(cand, nc, limit / 2, limit - limit / 8, lane, cap);
-        if (nc == 0 || nc > limit || !(*cap > 1.001f * t_lo + 1e-6f) || ++cuts > kMaxCuts) return -1;
+        if (nc == 0 || nc > limit || !(*cap > 1.001f * t_lo + 1e-6f) || ++cuts > (cull ? kMaxCuts : 6))
+          return -1;
       }
     }
   }
