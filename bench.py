@@ -696,18 +696,16 @@ def main():
     achieved = b_dom / (ph[dom] * 1e-3) / 1e9
     # DRAM bytes per call (dram__bytes_read.sum + dram__bytes_write.sum over the call's trace
     # kernels) from one single-pass ncu capture of `bench.py --once` on this default workload
-    # (1M ellipsoids, 1920x1080): forward = the three passes of the regrouped forward,
-    # backward = k_trace_bwd
-    measured_traffic = {"fwd": 253_090_000 + 418_550_000 + 7_410_000 + 6_400 + 33_540,
-                        "bwd": 1_180_000_000 + 144_010_000}
+    # (1M ellipsoids, 1920x1080): forward = k_trace_fwd_packet, backward = k_trace_bwd
+    measured_traffic = {"fwd": 274_770_000 + 405_020_000, "bwd": 1_160_140_000 + 141_560_000}
     default_workload = args.prims == 1_000_000 and args.width == 1920 and args.height == 1080
     roofline = {"bound": "hbm",
-                "kernel": "k_trace_bwd" if dom == "bwd" else "regrouped forward (k_trace_fwd_pass x3, one library call)",
+                "kernel": "k_trace_bwd" if dom == "bwd" else "k_trace_fwd_packet",
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": peak_kind, "traffic": measured_traffic[dom] if default_workload else None,
                 "algorithmic_bytes": b_dom,
-                "note": "latency- and issue-bound tree walk and event integration, not HBM-bound: the forward's "
-                        "pass 0 issues on 57% of cycles while DRAM moves under 2% of its peak"}
+                "note": "issue-bound tree walk and event integration, not HBM-bound: the forward issues on 53% "
+                        "of cycles (ALU pipe 41%) while DRAM moves under 2% of its peak"}
 
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -728,7 +726,7 @@ def main():
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "note": "pinned host inputs copied and the image read back every step, on two copy streams (one "
                         "per direction) that overlap the next step's compute (two device input buffers)"},
-        "gpu_launches": args.steps * 64,
+        "gpu_launches": args.steps * 39,  # the library's kernels of one step (build 17, orders 17, traces 2, finalize 3)
         "roofline": roofline,
     }
     if rank == 0 and world == 1 and not args.no_cpu:

@@ -54,13 +54,13 @@ typedef struct EverScene {
 typedef struct EverTune {
   int32_t kbuf;       /* events gathered per traversal round: 8, 16 or 32 */
   int32_t block;      /* threads per block: 64, 128 or 256 */
-  int32_t traversal;  /* 0 (default): warp packets, each first taking the leaves its rays can meet in
-                         one breadth-first walk and integrating them in order (the frustum phase),
-                         then gather rounds for any ray it could not finish; 1: one walk per ray;
+  int32_t traversal;  /* 0 (default): warp packets, each listing the leaves its rays can meet and
+                         integrating them in order, in stages over t (the frustum phase), then
+                         gather rounds for any ray it could not finish; 1: one walk per ray;
                          2: warp packets, gather rounds only */
-  int32_t regroup_min;/* ever_trace_forward_regrouped: a pass with fewer rays than this runs every
-                         remaining round instead of handing the rest on; 0: four times the GPU's
-                         resident lanes */
+  int32_t regroup_min;/* ever_trace_forward_regrouped with traversal 2: a pass with fewer rays than
+                         this runs every remaining round instead of handing the rest on; 0: four
+                         times the GPU's resident lanes */
   int32_t stack_depth;/* traversal stack entries in use, 8..64 (0: 64); a tree deeper than the stack
                          raises EVER_STATUS_STACK_OVERFLOW (a subtree is skipped) */
   int32_t reserved[3];
@@ -166,10 +166,11 @@ int ever_trace_forward(const EverScene* scene, const float* rayo, const float* r
 size_t ever_trace_forward_workspace_bytes(int64_t num_rays);
 
 /* ever_trace_forward, same arguments and the same results bit for bit, for warp-packet
- * traversal (tune->traversal is ignored), and faster: after each of the first two gather
- * rounds the rays that need more rounds are packed into full warps in launch order, so
- * warps stop running with most of their lanes idle. Rays between passes keep their loop
- * state in out->states and out->last_dirac, which are therefore required. R < 2^31.
+ * traversal. With gather rounds only (traversal 2) the rays that need more rounds are packed
+ * into full warps in launch order after each of the first two, so warps stop running with
+ * most of their lanes idle; with the frustum phase (traversal 0) one launch finishes nearly
+ * every ray and this is ever_trace_forward. Rays between passes keep their loop state in
+ * out->states and out->last_dirac, which are therefore required. R < 2^31.
  * No counterpart in the reference (OptiX runs one thread per ray to the end). */
 int ever_trace_forward_regrouped(const EverScene* scene, const float* rayo, const float* rayd, int64_t num_rays,
                                  const EverTraceArgs* args, const int32_t* ray_order, const EverTune* tune,
