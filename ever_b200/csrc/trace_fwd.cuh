@@ -572,7 +572,7 @@ constexpr int kCandCap = kStageLeaves + 64;
 // wide packets of small views cut too long (batched views 4.4 -> 5.0 ms).
 constexpr int kMaxCuts = 16;
 constexpr int kMaxStages = 128;  // then the rounds take over
-constexpr int kTileWords = 24;
+constexpr int kTileWords = 28;
 constexpr int kStateWords = 14;  // of a lane's integration state: State (13), the last event's id
 // Shared ints per warp: the walk's nodes with their entry bounds (before and after it, the
 // traversal stack of the rounds; after it, the events' ring),
@@ -614,6 +614,7 @@ struct PacketTile {
   float e1[3];     //   d0 + a e1 + b e2 with |a|, |b| <= 1
   float e2[3];
   float omin[3], omax[3], dmin[3], dmax[3];  // free axes only
+  float shift[3];  // how far rounding may have put a ray's start off its line; 0 with tmin = 0
 };
 static_assert(sizeof(PacketTile) <= kTileWords * sizeof(int), "tile words");
 
@@ -641,12 +642,15 @@ __device__ __forceinline__ PacketBounds packet_bounds(const Ray& ray, const RayS
     P.o_far[a] = neg ? omax : omin;
     common = common && amin == amax;
     m[a] = 0.5f * (dmin + dmax);
+    // a start that is not the apex itself is rounded to half an ulp (2^-24 of its size), twice that here
+    const float shift = 1.2e-7f * warp_max(part && o[a] != ap[a] ? fabsf(o[a]) : 0.f);
     if (lane == 0) {
       tile->o[a] = amin;
       tile->omin[a] = omin;
       tile->omax[a] = omax;
       tile->dmin[a] = dmin;
       tile->dmax[a] = dmax;
+      tile->shift[a] = shift;
     }
   }
   // tangent plane of the middle direction, and the rays' rectangle in it: the smallest over a
@@ -752,8 +756,13 @@ __device__ __forceinline__ float packet_entry(const PacketBounds& P, const Packe
 // v1, v2 normal to v0, s' = s / (1 + a p1 + b p2): a parallelogram, once s' is replaced by
 // its largest value. A ray's distance from the centre is at least its crossing point's
 // times the cosine of its angle to v0, so the packet misses when the parallelogram stays
-// farther than 1 / cos from the centre. The margins cover the float rounding here and in
-// the exact test (both about 1e-6 |c| of the radius); NaN never rejects.
+// farther than 1 / cos from the centre. In place of the radius 1 stands `rad`, which covers the
+// float rounding of the exact test and of this one. Both work with W (x - mean), whose
+// component i carries a few roundings of sum_a |W_ia| |x_a - mean_a| (about 18 times 2^-24 in
+// all; 2e-6 is 33), which for a turned thin ellipsoid can be far more than the component;
+// the roots along the ray add about 10 times 2^-24 of |c|. The exact test starts at the rounded
+// rayo + tmin rayd, which lies off the ray's line by tile->shift: by as much as the coordinates
+// are large, however near the ellipsoid. NaN never rejects.
 __device__ __forceinline__ bool packet_misses(const PacketTile* T, const Record* __restrict__ recs, int j) {
   const float4* rp = reinterpret_cast<const float4*>(recs + j);
   const float4 r[3] = {__ldg(rp), __ldg(rp + 1), __ldg(rp + 2)};
@@ -794,8 +803,12 @@ __device__ __forceinline__ bool packet_misses(const PacketTile* T, const Record*
     f = fminf(f, fmaf(a, fmaf(a, C11, 2.f * h1), fmaf(2.f * sg, B2, A + C22)));
     f = fminf(f, fmaf(b, fmaf(b, C22, 2.f * h2), fmaf(2.f * sg, B1, A + C11)));
   }
-  const float size = fabsf(c[0]) + fabsf(c[1]) + fabsf(c[2]);
-  const float lim = (1.f + tan2) * (1.002f + 1e-5f * size) + 4e-6f * (A + C11 + C22);
+  const float ex = fmaf(2e-6f, fabsf(x), T->shift[0]), ey = fmaf(2e-6f, fabsf(y), T->shift[1]),
+              ez = fmaf(2e-6f, fabsf(z), T->shift[2]);
+  float rad = fmaf(5e-6f, fabsf(c[0]) + fabsf(c[1]) + fabsf(c[2]), 1.001f);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) rad = fmaf(fabsf(r[i].z), ez, fmaf(fabsf(r[i].y), ey, fmaf(fabsf(r[i].x), ex, rad)));
+  const float lim = (1.f + tan2) * (rad * rad) + 4e-6f * (A + C11 + C22);
   return g < 0.5f && !inside && f > lim && C11 + C22 < 1e5f;
 }
 
