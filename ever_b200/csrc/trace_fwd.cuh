@@ -1249,7 +1249,7 @@ __device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx
     }
     const LeafList list = list_leaves(sc.nodes, sc.recs, ray.o, ray.d, ray.apex, mine, t_lo, cap,
                                       t_lo == 0.f ? kFirstLeaves : kStageLeaves, at, lane);
-    const int nc = list.n;
+    int nc = list.n;
     const bool cut = list.cap < cap;
     cap = list.cap;
     // half a group's lanes cover as much as all did: directions in no order, for the rounds
@@ -1267,6 +1267,9 @@ __device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx
     }
     // events from `end` on belong to the next stage
     const uint64_t end = uint64_t(cap < cap_all ? __float_as_uint(cap) : 0x7f800000u) << 32;
+    // A leaf whose bound lies at or past the cut (the walk's margins list a few) has no event
+    // before it, and must not raise T past it: a leaf left off the list may come first there.
+    while (nc > 0 && cand[nc - 1] >= end) --nc;
     // Passes over the list: one, unless a lane's buffer overflows. It then keeps its smallest
     // events and takes those; the events from `over` (the smallest it dropped) on are
     // collected again by another pass.
