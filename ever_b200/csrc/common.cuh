@@ -45,9 +45,6 @@ __device__ __forceinline__ float safe_div(float a, float b) {
 __device__ __forceinline__ float safe_exp(float v) { return expf(clampf(v, kMinVal, kLogMax)); }
 __device__ __forceinline__ float sgnf(float x) { return x > 0.f ? 1.f : (x < 0.f ? -1.f : 0.f); }
 
-// 1 / x as safe_div takes it: the denominator's magnitude is kept from kTiny down.
-__device__ __forceinline__ float safe_rcp(float x) { return 1.f / (fabsf(x) < kTiny ? kTiny : x); }
-
 // tukey_power_ladder(x, -0.1), safe-math.slang:246-253
 __device__ __forceinline__ float tukey(float x) {
   const float p = -0.1f;

@@ -84,10 +84,9 @@ __device__ __forceinline__ Ctrl load_ctrl(const Record* recs, const float* feats
 // and G, the cotangent of the state after, that of the state before (the VJP of update()).
 // Both share their terms: the weight, the colours and the distance warp are evaluated once.
 // Clamps pass the gradient only strictly inside their range (a zero-density gap gets none);
-// safe_div's backward as safe-math.slang:68-80, its six quotients by two reciprocals (they
-// reach the density and feature gradients only; the colours and the warp, whose terms cancel
-// in the event times' gradients, keep their divisions and powers). The colour sum C is not
-// undone: nothing reads it. Outputs: Gt, Gdirac.
+// safe_div's backward as safe-math.slang:68-80. An event without weight (w R = 0 below: a gap)
+// needs none of the quotients, whose slowest case is 0 / 0. The colour sum C is not undone:
+// nothing reads it. Outputs: Gt, Gdirac.
 __device__ __forceinline__ void step_back(State& n, State& G, float t, float4 dirac, float t_old, float& Gt,
                                           float4& Gdirac) {
   const float dt_raw = t - t_old;
@@ -95,11 +94,7 @@ __device__ __forceinline__ void step_back(State& n, State& G, float t, float4 di
   const float4 d = make_float4(n.drgb.x - dirac.x, n.drgb.y - dirac.y, n.drgb.z - dirac.z, n.drgb.w - dirac.w);
   const float area_raw = d.x * dt;
   const float area = fmaxf(area_raw, 0.f);
-  const float inv = safe_rcp(d.x);
   const float dv[3] = {d.y, d.z, d.w};
-  float rgb[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) rgb[i] = safe_div(dv[i], d.x);
   const float logT = fmaxf(n.logT - area, 0.f);
   const float ea_in = -area, el_in = -logT;
   const float e1 = safe_exp(ea_in), e2 = safe_exp(el_in);
@@ -116,23 +111,28 @@ __device__ __forceinline__ void step_back(State& n, State& G, float t, float4 di
   float g_area = area + logT > 0.f ? G.logT : 0.f;
   float GslogT = g_area;
   const float Gc[3] = {G.C.x, G.C.y, G.C.z};
-  float g_w = Gc[0] * rgb[0] + Gc[1] * rgb[1] + Gc[2] * rgb[2];
+  float g_w = 0.f;
+  if (wraw > 0.f && wraw < 1.f)
+    g_w = Gc[0] * safe_div(dv[0], d.x) + Gc[1] * safe_div(dv[1], d.x) + Gc[2] * safe_div(dv[2], d.x);
   g_w += G.dist_x * 2.f * m * cum_x + G.dist_y * 2.f * cum_y + G.cum_x + G.cum_y * m;
   const float g_m = G.dist_x * 2.f * w * cum_x + G.cum_y * w;
   G.cum_x = G.cum_x + G.dist_x * 2.f * w * m;
   G.cum_y = G.cum_y + G.dist_y * 2.f * w;
-  const float b2 = d.x * d.x, inv2 = 1.f / (b2 < kTiny ? kTiny : b2);
-  float gd[3], gx = 0.f;
+  const float R[3] = {Gc[0] * w, Gc[1] * w, Gc[2] * w};
+  float gd[3] = {0.f, 0.f, 0.f}, gx = 0.f;
+  if (R[0] != 0.f || R[1] != 0.f || R[2] != 0.f) {
+    const float b2 = d.x * d.x, den = fabsf(d.x) < kTiny ? kTiny : d.x, den2 = b2 < kTiny ? kTiny : b2;
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const float R = Gc[i] * w;
-    gd[i] = clampf(R * inv, kMinVal, kMaxVal);
-    gx += clampf((-dv[i] * inv2) * R, kMinVal, kMaxVal);
+    for (int i = 0; i < 3; ++i) {
+      gd[i] = clampf(R[i] / den, kMinVal, kMaxVal);
+      gx += clampf((-dv[i] / den2) * R[i], kMinVal, kMaxVal);
+    }
   }
   if (wraw > 0.f && wraw < 1.f) {
     if (ea_in > kMinVal && ea_in < kLogMax) g_area += g_w * e2 * e1;
     if (el_in > kMinVal && el_in < kLogMax) GslogT += -g_w * (1.f - e1) * e2;
   }
+  gx = Gdirac.x + gx;
   if (area_raw > 0.f) {
     gx += g_area * dt;
     const float g_dt = g_area * d.x;
@@ -145,7 +145,7 @@ __device__ __forceinline__ void step_back(State& n, State& G, float t, float4 di
   const float g_mid = g_m * dm * 500.f;
   Gt += g_mid;
   Gst += g_mid;
-  G.drgb = make_float4(Gdirac.x + gx, Gdirac.y + gd[0], Gdirac.z + gd[1], Gdirac.w + gd[2]);
+  G.drgb = make_float4(gx, Gdirac.y + gd[0], Gdirac.z + gd[1], Gdirac.w + gd[2]);
   G.logT = GslogT;
   G.t = Gst;
   n.drgb = d;

@@ -1,5 +1,6 @@
-"""The colour quotients of an event are IEEE divisions: with one opaque ellipsoid per ray (weight
-exactly 1) the image equals the same float32 operations in numpy, bit for bit."""
+"""The colour quotients of an event and their derivatives are IEEE divisions: with one opaque
+ellipsoid per ray (weight exactly 1) the image, the feature gradients and the density gradients
+equal the same float32 operations in numpy, bit for bit."""
 import numpy as np
 import pytest
 import torch
@@ -37,3 +38,16 @@ def _traced(traversal):
 def test_colours_are_the_quotients(traversal):
     fwd, _, _, _, _, sigma, sc, _ = _traced(traversal)
     assert np.array_equal(fwd.out[:, :3].cpu().numpy(), sc / sigma)
+
+
+def test_gradients_are_the_quotients():
+    fwd, scene, ro, rd, t, sigma, sc, colour = _traced(0)
+    g = np.random.default_rng(4).standard_normal((N, 3)).astype(np.float32)
+    grad = np.concatenate([g, np.zeros((N, 2))], 1)
+    got = T.backward(scene, ro, rd, fwd, t(grad))
+    gd = g / sigma  # d loss / d (density * colour) before the exit
+    assert np.array_equal(got.features[:, 0].cpu().numpy(), np.clip(C0 * (sigma * gd), -1e3, 1e3))
+    gx = ((-sc) / (sigma * sigma)) * g
+    gx = (gx[:, 0] + gx[:, 1]) + gx[:, 2]
+    want = ((gx + gd[:, 0] * colour[:, 0]) + gd[:, 1] * colour[:, 1]) + gd[:, 2] * colour[:, 2]
+    assert np.array_equal(got.density.cpu().numpy(), np.clip(want, -50, 50))
