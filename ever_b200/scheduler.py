@@ -25,6 +25,7 @@ from typing import Optional, Sequence
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from . import _native as N
 
@@ -176,15 +177,34 @@ def cost_targets(ray_stats: torch.Tensor, rayo: torch.Tensor, rayd: torch.Tensor
     return t
 
 
+def _one_kernel(pred, rayo, rayd, centre, scale, out) -> bool:
+    """Whether depth_from_prediction may run as the library's kernel: plain float32 CUDA arrays
+    of the usual shapes that nothing traces, maps or differentiates, three numbers for the
+    centre and one for the scale. Everything else is the torch expression's."""
+    if torch.compiler.is_compiling() or not isinstance(scale, (int, float)):
+        return False
+    if not isinstance(centre, (tuple, list)) or len(centre) != 3 or not all(isinstance(v, (int, float)) for v in centre):
+        return False
+    ts = (pred, rayo, rayd) + (() if out is None else (out,))
+    if any(type(t) is not torch.Tensor or torch._C._functorch.is_functorch_wrapped_tensor(t) for t in ts):
+        return False
+    if not all(t.is_cuda and t.device == pred.device and t.dtype == torch.float32 and t.is_contiguous()
+               and not t.is_neg() and not t.requires_grad and forward_ad.unpack_dual(t).tangent is None for t in ts):
+        return False
+    R = rayo.shape[0]
+    if not rayo.shape == rayd.shape == (R, 3) or pred.shape != (R, 2) or R >= 1 << 31:
+        return False
+    # the kernel writes a ray's hint while other rays are read
+    return out is None or (out.shape == (R,) and all(out.untyped_storage().data_ptr() != t.untyped_storage().data_ptr()
+                                                     for t in ts[:3]))
+
+
 def depth_from_prediction(pred: torch.Tensor, rayo: torch.Tensor, rayd: torch.Tensor, centre=(0.0, 0.0, 0.0),
                           scale: float = 1.0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """(R,) stopping t guessed by the model (the inverse of cost_targets' depth column): the
     depth hint the tracer's frustum phase takes (tracer.forward(depth_hint=...))."""
-    ts = (pred, rayo, rayd) + (() if out is None else (out,))
     R = rayo.shape[0]
-    if (all(t.is_cuda and t.device == pred.device and t.dtype == torch.float32 and t.is_contiguous()
-            and not t.requires_grad for t in ts)
-            and rayo.shape == rayd.shape == (R, 3) and pred.shape == (R, 2) and (out is None or out.shape == (R,))):
+    if _one_kernel(pred, rayo, rayd, centre, scale, out):
         d = torch.empty(R, dtype=torch.float32, device=pred.device) if out is None else out
         with torch.cuda.device(pred.device):
             N.check(N.load().ever_depth_hint(N.ptr(pred), N.ptr(rayo), N.ptr(rayd), R,
