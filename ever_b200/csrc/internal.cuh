@@ -75,6 +75,12 @@ struct FwdParams {
   int stack_depth;  // traversal stack entries in use, <= kStackDepth (set from the tune)
   int lanes;        // frustum kernels: rays per packet, <= 32 (set by the launcher)
   const float* depth_hint;  // (R) nullable: per-ray guess of the stopping t (first frustum stage)
+  // A launch whose rays may come in no order: the sampled packets in which they do are counted
+  // in *votes, and from vote_min on the gather rounds trace the launch (taking packets from
+  // *taken) instead of the frustum kernel. Device words; null: no vote.
+  uint32_t* votes;
+  uint32_t* taken;
+  uint32_t vote_min;
 };
 
 cudaError_t launch_forward(const FwdParams& P, int deg, const EverTune& tune, cudaStream_t st);

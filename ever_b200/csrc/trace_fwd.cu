@@ -132,11 +132,15 @@ cudaError_t launch_forward_regrouped(const FwdParams& P0, const RegroupScratch& 
   const FwdParams P = with_mode(P0, tune);
   if (P.R == 0) return cudaSuccess;
   const int block = tune.block > 0 ? tune.block : 128;
-  // the frustum phase finishes nearly every ray in one launch: nothing to pack again
+  // the frustum phase finishes nearly every ray of ordered packets in one launch: nothing to pack
+  // again; ray arrays in no order are for the rounds (a camera's tiles are always in order)
   if (P.frustum) {
     EverTune t = tune;
     t.traversal = 0;
-    return cam ? launch_forward_camera(P, *cam, jitter, deg, t, st) : launch_forward(P, deg, t, st);
+    FwdParams F = P;
+    F.votes = W.count1;
+    F.taken = W.count2;
+    return cam ? launch_forward_camera(P, *cam, jitter, deg, t, st) : launch_forward(F, deg, t, st);
   }
   // splitting pays only while the next pass still fills the GPU several times over: four
   // times the resident lanes of the packet kernels (20 warps per SM)

@@ -1441,6 +1441,7 @@ struct FwdMinBlocks {
 template <int KBUF, int DEG, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK>::value) k_trace_fwd_packet(const FwdParams P) {
   extern __shared__ int smem[];
+  if (P.votes && __ldg(P.votes) >= P.vote_min) return;  // the rounds trace this launch
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int* wstack = smem + warp * kWarpInts;  // traversal stack, and the frustum phase's lists over it
   float* B = reinterpret_cast<float*>(smem + (blockDim.x / 32) * kWarpInts) + tid;  // B[k * blockDim.x]
@@ -1524,6 +1525,63 @@ __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK, false>::value)
   }
 }
 
+// Rays in no order (random rays, shuffled pixels, the sorted pixels of many views) are traced by
+// the gather rounds. Inside the frustum kernel these have 16 warps per SM and the L1 that the
+// lists leave; in their own kernel 20 and nearly all of it: 262,144 random rays against 20,000
+// ellipsoids 13.7 and 9.1 ms, against 300,000 22.7 and 15.6 ms; random pixels of 100 views 13.8
+// and 8.6 ms. So one block looks at up to kVotePackets full packets, evenly spaced, and counts
+// those in no order. More than half of them: the rounds take the launch. A launch with fewer
+// (pixels of 8 views: an eighth) is the frustum kernel's, whose own rounds overlap with its
+// other packets. The vote takes 6 us (256 packets in its block: 15) and the
+// empty second launch 2.
+constexpr uint32_t kVotePackets = 64;
+__global__ void __launch_bounds__(1024) k_order_vote(const FwdParams P, uint32_t packets) {
+  __shared__ uint32_t votes;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) votes = 0;
+  __syncthreads();
+  uint32_t n = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kVotePackets / 32; ++q) {
+    const uint32_t v = 32 * q + threadIdx.x / 32;
+    if (v >= packets) break;
+    const int64_t gi = P.R / 32 * v / packets * 32 + lane;  // full packets only
+    n += no_order(load_ray(P.rayo, P.rayd, P.ray_order ? int64_t(P.ray_order[gi]) : gi, P.tmin), kFull, lane) ? 1u : 0u;
+  }
+  if (lane == 0 && n) atomicAdd(&votes, n);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *P.votes = votes;
+    *P.taken = 0;
+  }
+}
+
+// The rounds of a launch in no order. Persistent (an empty launch of one block per packet takes
+// 10 us at full HD): warps take packets from a device counter.
+constexpr int kUnorderedBlock = 128;
+template <int KBUF, int DEG>
+__global__ void __launch_bounds__(kUnorderedBlock, FwdMinBlocks<kUnorderedBlock, false>::value)
+    k_trace_fwd_unordered(const FwdParams P) {
+  extern __shared__ int smem[];
+  if (__ldg(P.votes) < P.vote_min) return;  // the frustum kernel has traced this launch
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int* wstack = smem + warp * kStackDepth;
+  float* B = reinterpret_cast<float*>(smem + (kUnorderedBlock / 32) * kStackDepth) + tid;
+  const SceneRef sc = scene_of(P);
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
+  for (;;) {
+    uint32_t packet = 0;
+    if (lane == 0) packet = atomicAdd(P.taken, 1u);
+    packet = __shfl_sync(kFull, packet, 0);
+    const int64_t gi = int64_t(packet) * 32 + lane;
+    if (int64_t(packet) * 32 >= P.R) break;
+    const bool valid = gi < P.R;
+    const int64_t r = valid ? (P.ray_order ? int64_t(P.ray_order[gi]) : gi) : 0;
+    const Ray ray = load_ray(P.rayo, P.rayd, r, P.tmin);
+    trace_packet<KBUF, DEG, false>(sc, C, ray, r, valid, gi, wstack, B, kUnorderedBlock, lane);
+  }
+}
+
 // Camera trace: rays are made from the camera in the kernel (no ray arrays). The launch
 // covers the camera's slots, 32 per 8x4 pixel tile, so a warp traces one tile; outputs are
 // written by pixel, event-log columns are slots.
@@ -1603,6 +1661,28 @@ inline int packet_lanes(int64_t rays) {
   return lanes;
 }
 
+// The vote of a launch of full packets. Narrow packets (launches that leave warps idle) have
+// none: theirs is the frustum kernel, and two more launches would cost them (2 us each).
+inline cudaError_t vote_begin(FwdParams& P, cudaStream_t st) {
+  const uint32_t packets = uint32_t(std::min<int64_t>(P.R / 32, kVotePackets));
+  if (P.lanes < 32 || packets == 0) P.votes = nullptr;
+  if (!P.votes) return cudaSuccess;
+  P.vote_min = packets / 2 + 1;
+  k_order_vote<<<1, 1024, 0, st>>>(P, packets);
+  return cudaGetLastError();
+}
+template <int KBUF, int DEG>
+cudaError_t vote_finish(const FwdParams& P, cudaStream_t st) {
+  if (!P.votes) return cudaGetLastError();
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const size_t smem = packet_smem<DEG>(kUnorderedBlock, false);
+  if (cudaError_t e_ = prepare(k_trace_fwd_unordered<KBUF, DEG>, smem)) return e_;
+  k_trace_fwd_unordered<KBUF, DEG>
+      <<<sms * FwdMinBlocks<kUnorderedBlock, false>::value, kUnorderedBlock, smem, st>>>(P);
+  return cudaGetLastError();
+}
+
 // Gather rounds only, one pass that runs them all.
 template <int KBUF, int DEG, int BLOCK, bool CAM>
 cudaError_t launch_rounds_b(const FwdParams& P, const PassCamera& Q, cudaStream_t st) {
@@ -1636,6 +1716,7 @@ cudaError_t launch_t(const FwdParams& P0, int block, int traversal, cudaStream_t
   } else if (traversal == 2) {
     return launch_rounds<KBUF, DEG, false>(P, PassCamera{}, block, st);
   } else {
+    if (cudaError_t e_ = vote_begin(P, st)) return e_;
     const size_t smem = packet_smem<DEG>(block);
     switch (block) {
       case 64: {
@@ -1654,6 +1735,7 @@ cudaError_t launch_t(const FwdParams& P0, int block, int traversal, cudaStream_t
         break;
       }
     }
+    return vote_finish<KBUF, DEG>(P, st);
   }
   return cudaGetLastError();
 }

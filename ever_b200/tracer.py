@@ -163,10 +163,11 @@ def forward(scene: Scene, rayo, rayd, tmin=0.0, tmax=1000.0, max_iters=500, sh_d
             touch_count=False, ray_stats=False, ray_order=None, tune: Tune | None = None,
             buffers: ForwardResult | None = None, regrouped: bool = True,
             workspace: torch.Tensor | None = None, depth_hint: torch.Tensor | None = None) -> ForwardResult:
-    """regrouped: with warp packets (tune.traversal 0) and k-buffers of up to 16 events,
-    re-pack the rays that need more gather rounds into full warps between passes
-    (ever_trace_forward_regrouped; same results, faster). workspace: optional uint8 scratch
-    of ever_trace_forward_workspace_bytes(R)."""
+    """regrouped: with warp packets (tune.traversal 0 or 2) and k-buffers of up to 16 events, run
+    ever_trace_forward_regrouped: same results; with traversal 2 the rays that need more gather
+    rounds are packed into full warps between passes, with traversal 0 a launch whose rays come
+    in no order runs the rounds in a kernel of their own. workspace: optional uint8 scratch of
+    ever_trace_forward_workspace_bytes(R)."""
     device = scene.device
     _check_tensor("ray_origins", rayo, device, 3)
     _check_tensor("ray_directions", rayd, device, 3)
@@ -204,8 +205,8 @@ def forward(scene: Scene, rayo, rayd, tmin=0.0, tmax=1000.0, max_iters=500, sh_d
     tune = tune or Tune()
     lib = N.load()
     with on_device(device):
-        # the packed passes pay for buffers of up to 16 events; with 32, most rays finish in
-        # the first round and the extra passes only add their overhead
+        # the packed passes of traversal 2 pay for buffers of up to 16 events; with 32, most rays
+        # finish in the first round and the extra passes only add their overhead
         if regrouped and tune.traversal in (0, 2) and tune.kbuf <= 16 and R < (1 << 31):
             need = int(lib.ever_trace_forward_workspace_bytes(R))
             if workspace is None or workspace.numel() < need:

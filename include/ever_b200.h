@@ -168,9 +168,11 @@ size_t ever_trace_forward_workspace_bytes(int64_t num_rays);
 /* ever_trace_forward, same arguments and the same results bit for bit, for warp-packet
  * traversal. With gather rounds only (traversal 2) the rays that need more rounds are packed
  * into full warps in launch order after each of the first two, so warps stop running with
- * most of their lanes idle; with the frustum phase (traversal 0) one launch finishes nearly
- * every ray and this is ever_trace_forward. Rays between passes keep their loop state in
- * out->states and out->last_dirac, which are therefore required. R < 2^31.
+ * most of their lanes idle. With the frustum phase (traversal 0) nothing is packed; a launch that
+ * fills the GPU first looks whether its rays come in any order (64 of its packets), and if
+ * not traces them with gather rounds in a kernel of their own. Traversal 1: as 2 where a
+ * launch is large enough to split (regroup_min), else as 0. Rays between passes keep their
+ * loop state in out->states and out->last_dirac, which are therefore required. R < 2^31.
  * No counterpart in the reference (OptiX runs one thread per ray to the end). */
 int ever_trace_forward_regrouped(const EverScene* scene, const float* rayo, const float* rayd, int64_t num_rays,
                                  const EverTraceArgs* args, const int32_t* ray_order, const EverTune* tune,
