@@ -61,6 +61,17 @@ def workload(args, rank=0):
     return sc, ro, rd
 
 
+def step_launches(prims, rays, sms=148):
+    """Kernels of the library in one step (build, ray order, forward, backward order, backward) of
+    a DC-colour trace with feature rows."""
+    def sort(n, passes):  # one launch up to 8,192 keys, then two a pass up to 16 tiles of 2,048, three beyond
+        return 1 if n <= 8192 else passes * (2 if n <= 16 * 2048 else 3)
+    build = 5 + sort(prims, 4)  # boxes, keys, gather, tree, refit
+    orders = 2 + sort(rays, 4) + sort(rays, 1)
+    traces = 4 if rays > sms * 16 * 16 else 2  # full packets: the order's vote and the rounds it may call
+    return build + orders + traces + 3  # finalize: inverse order, geometry, features
+
+
 def workload_name(args):
     return (f"{args.prims} clustered ellipsoids SH3, {args.width}x{args.height} rays, "
             f"forward+backward via torch.autograd (BVH build per step)")
@@ -704,8 +715,9 @@ def main():
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": peak_kind, "traffic": measured_traffic[dom] if default_workload else None,
                 "algorithmic_bytes": b_dom,
-                "note": "issue-bound tree walk and event integration, not HBM-bound: the forward issues on 53% "
-                        "of cycles (ALU pipe 41%) while DRAM moves under 2% of its peak"}
+                "note": "issue-bound tree walk and event integration, not HBM-bound"
+                        + (": the forward issues on 53% of cycles (ALU pipe 41%) while DRAM moves under 2% of its "
+                           "peak" if default_workload else "")}
 
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -726,7 +738,7 @@ def main():
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "note": "pinned host inputs copied and the image read back every step, on two copy streams (one "
                         "per direction) that overlap the next step's compute (two device input buffers)"},
-        "gpu_launches": args.steps * 39,  # the library's kernels of one step (build 17, orders 17, traces 2, finalize 3)
+        "gpu_launches": args.steps * step_launches(N, R),
         "roofline": roofline,
     }
     if rank == 0 and world == 1 and not args.no_cpu:
