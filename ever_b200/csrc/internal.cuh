@@ -26,12 +26,15 @@ struct SceneLayout {
   int64_t nodes, records, features, order;
   int64_t aabb_a, aabb_b, keys_a, keys_b, vals_a, vals_b, hist;
   int64_t parent_node, parent_leaf, flags, bounds;
-  int nblocks;
   int64_t total;
 };
 
 SceneLayout scene_layout(int64_t N, int K);
-int sort_blocks(int64_t N);
+// Radix sort scratch: a histogram of 256 words for each tile of kSortTile keys, then the digits'
+// totals (256 words; the rest keeps the workspace sizes callers may have stored).
+constexpr int kSortTile = 2048, kSortExtra = 512;
+constexpr int64_t sort_blocks(int64_t N) { return ((N > 1 ? N : 1) + kSortTile - 1) / kSortTile; }
+constexpr int64_t sort_hist_bytes(int64_t N) { return (sort_blocks(N) * 256 + kSortExtra) * int64_t(sizeof(uint32_t)); }
 void sort_pairs(uint32_t*& ka, uint32_t*& va, uint32_t*& kb, uint32_t*& vb, uint32_t* hist, int64_t N, int bits,
                 cudaStream_t st);
 int64_t ray_order_workspace(int64_t R);

@@ -150,7 +150,7 @@ cudaError_t camera_backward_slot_order(const CameraParams& cam, const int32_t* i
   uint32_t* va = reinterpret_cast<uint32_t*>(ws + c.take(S * 4));
   uint32_t* kb = reinterpret_cast<uint32_t*>(ws + c.take(S * 4));
   uint32_t* vb = reinterpret_cast<uint32_t*>(ws + c.take(S * 4));
-  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + c.take((int64_t(sort_blocks(S)) * 256 + 512) * 4));
+  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + c.take(sort_hist_bytes(S)));
   k_camera_bwd_keys<<<unsigned((S + 255) / 256), 256, 0, st>>>(cam, iters, S, shift, ka, va);
   sort_pairs(ka, va, kb, vb, hist, S, 8, st);
   return cudaMemcpyAsync(slot_order, va, S * sizeof(int32_t), cudaMemcpyDeviceToDevice, st);
@@ -164,7 +164,7 @@ cudaError_t backward_slot_order(const int32_t* iters, const int32_t* ray_order, 
   uint32_t* va = reinterpret_cast<uint32_t*>(ws + c.take(R * 4));
   uint32_t* kb = reinterpret_cast<uint32_t*>(ws + c.take(R * 4));
   uint32_t* vb = reinterpret_cast<uint32_t*>(ws + c.take(R * 4));
-  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + c.take((int64_t(sort_blocks(R)) * 256 + 512) * 4));
+  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + c.take(sort_hist_bytes(R)));
   k_bwd_keys<<<unsigned((R + 255) / 256), 256, 0, st>>>(iters, ray_order, R, shift, views, num_views, ka, va);
   sort_pairs(ka, va, kb, vb, hist, R, views ? 14 : 8, st);
   return cudaMemcpyAsync(slot_order, va, R * sizeof(int32_t), cudaMemcpyDeviceToDevice, st);
@@ -180,7 +180,7 @@ cudaError_t batch_ray_order(const float* rayo, const float* rayd, int64_t R, con
   uint32_t* va = reinterpret_cast<uint32_t*>(ws + c.take(R * 4));
   uint32_t* kb = reinterpret_cast<uint32_t*>(ws + c.take(R * 4));
   uint32_t* vb = reinterpret_cast<uint32_t*>(ws + c.take(R * 4));
-  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + c.take((int64_t(sort_blocks(R)) * 256 + 512) * 4));
+  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + c.take(sort_hist_bytes(R)));
   k_batch_ray_keys<<<unsigned((R + 255) / 256), 256, 0, st>>>(rayd, R, views, num_views, bins, ka, va);
   sort_pairs(ka, va, kb, vb, hist, R, bins ? 32 : 30, st);
   k_batch_fill_slots<<<unsigned((R + 255) / 256), 256, 0, st>>>(va, R, views, num_views, slot_ray);
@@ -193,7 +193,7 @@ int64_t ray_order_workspace(int64_t R) {
   c.take(R * 4);
   c.take(R * 4);
   c.take(R * 4);
-  c.take((int64_t(sort_blocks(R)) * 256 + 512) * 4);
+  c.take(sort_hist_bytes(R));
   return c.offset;
 }
 
@@ -205,7 +205,7 @@ cudaError_t ray_order(const float* rayo, const float* rayd, int64_t R, char* ws,
   uint32_t* va = reinterpret_cast<uint32_t*>(ws + c.take(R * 4));
   uint32_t* kb = reinterpret_cast<uint32_t*>(ws + c.take(R * 4));
   uint32_t* vb = reinterpret_cast<uint32_t*>(ws + c.take(R * 4));
-  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + c.take((int64_t(sort_blocks(R)) * 256 + 512) * 4));
+  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + c.take(sort_hist_bytes(R)));
   k_ray_keys<<<unsigned((R + 255) / 256), 256, 0, st>>>(rayo, rayd, R, bins, ka, va);
   sort_pairs(ka, va, kb, vb, hist, R, bins ? 32 : 30, st);
   return cudaMemcpyAsync(order, va, R * sizeof(int32_t), cudaMemcpyDeviceToDevice, st);

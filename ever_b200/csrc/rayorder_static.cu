@@ -30,9 +30,9 @@ namespace {
 
 constexpr int64_t kStaticOrderMaxRays = int64_t(1) << 21;  // 2,097,152 rays
 constexpr int64_t round256(int64_t b) { return (b + 255) / 256 * 256; }
-// Same segment layout as ray_order_workspace(): keys, values, keys, values, histogram + scan partials.
+// Same segment layout as ray_order_workspace(): keys, values, keys, values, histogram.
 constexpr int64_t kStaticOrderBytes =
-    4 * round256(kStaticOrderMaxRays * 4) + round256(((kStaticOrderMaxRays + 2047) / 2048 * 256 + 512) * 4);
+    4 * round256(kStaticOrderMaxRays * 4) + round256(sort_hist_bytes(kStaticOrderMaxRays));
 
 static __device__ __align__(256) unsigned char g_order_scratch[kStaticOrderBytes];
 

@@ -16,8 +16,7 @@ namespace ever {
 namespace {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 8;
-constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr int kSortItems = kSortTile / kSortThreads;
 constexpr int kSortWarps = kSortThreads / 32;
 
 __device__ __forceinline__ uint32_t float_to_ordered(float f) {
@@ -194,7 +193,6 @@ __global__ void k_sort_hist(const uint32_t* __restrict__ keys, int64_t N, int sh
   hist[int64_t(threadIdx.x) * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
-constexpr int kScanChunks = 512;  // words after the histogram: digit totals (256 used)
 constexpr int kScanThreads = 256;
 
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* sh, uint32_t& total) {
@@ -582,11 +580,9 @@ void launch_gather_features(const int32_t* order, int64_t N, int K, const float*
 
 }  // namespace
 
-int sort_blocks(int64_t N) { return int(div_up(std::max<int64_t>(N, 1), kSortTile)); }
-
 // Stable LSD radix sort of (key, value) pairs on the low `bits` key bits, 8 bits per pass.
 // On return the sorted pairs are in (ka, va); (kb, vb) are scratch of the same size and
-// hist holds sort_blocks(N) * 256 words.
+// hist holds sort_hist_bytes(N).
 void sort_pairs(uint32_t*& ka, uint32_t*& va, uint32_t*& kb, uint32_t*& vb, uint32_t* hist, int64_t N, int bits,
                 cudaStream_t st) {
   if (N <= kSmallSort) {
@@ -597,8 +593,8 @@ void sort_pairs(uint32_t*& ka, uint32_t*& va, uint32_t*& kb, uint32_t*& vb, uint
     }
     cudaGetLastError();  // the general path needs no opt-in
   }
-  const int nblocks = sort_blocks(N);
-  uint32_t* totals = hist + int64_t(nblocks) * 256;  // within the kScanChunks words after the histogram
+  const int nblocks = int(sort_blocks(N));
+  uint32_t* totals = hist + int64_t(nblocks) * 256;
   const bool rows = nblocks > kDirectBlocks;
   for (int shift = 0; shift < bits; shift += 8) {
     k_sort_hist<<<nblocks, kSortThreads, 0, st>>>(ka, N, shift, hist, nblocks);
@@ -623,8 +619,7 @@ SceneLayout scene_layout(int64_t N, int K) {
   L.keys_b = c.take(N * sizeof(uint32_t));
   L.vals_a = c.take(N * sizeof(uint32_t));
   L.vals_b = c.take(N * sizeof(uint32_t));
-  L.nblocks = sort_blocks(N);
-  L.hist = c.take((int64_t(L.nblocks) * 256 + kScanChunks) * sizeof(uint32_t));
+  L.hist = c.take(sort_hist_bytes(N));
   L.parent_node = c.take(std::max<int64_t>(n1, 1) * sizeof(int32_t));
   L.parent_leaf = c.take(std::max<int64_t>(N, 1) * sizeof(int32_t));
   L.flags = c.take(std::max<int64_t>(n1, 1) * sizeof(uint32_t));
