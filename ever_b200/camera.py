@@ -124,9 +124,8 @@ def forward(scene: T.Scene, camera: Camera, jitter=None, tmin=0.0, tmax=1000.0, 
             log_events=True, touch_count=False, ray_stats=False, tune: T.Tune | None = None,
             regrouped: bool = True) -> T.ForwardResult:
     """Forward trace of the camera's pixels; results by pixel, event-log columns by slot.
-    regrouped: with gather rounds (tune.traversal 2) and k-buffers of up to 16 events, pack the
-    pixels still active after the first rounds into full warps
-    (ever_trace_forward_camera_regrouped; same results)."""
+    regrouped: with k-buffers of up to 16 events, pack the pixels still active after the
+    first gather rounds into full warps (ever_trace_forward_camera_regrouped; same results)."""
     device = scene.device
     R, S = camera.num_pixels, camera_slots(camera)
     jitter = _jitter(jitter, R, device)
@@ -150,7 +149,7 @@ def forward(scene: T.Scene, camera: Camera, jitter=None, tmin=0.0, tmax=1000.0, 
     tune = tune or T.Tune()
     lib = N.load()
     with on_device(device):
-        if regrouped and tune.traversal != 0 and tune.kbuf <= 16:
+        if regrouped and tune.kbuf <= 16:
             ws = torch.empty(max(int(lib.ever_trace_forward_workspace_bytes(S)), 256), dtype=torch.uint8,
                              device=device)
             N.check(lib.ever_trace_forward_camera_regrouped(ctypes.byref(scene.c), ctypes.byref(camera.c()),
