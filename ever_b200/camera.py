@@ -124,8 +124,10 @@ def forward(scene: T.Scene, camera: Camera, jitter=None, tmin=0.0, tmax=1000.0, 
             log_events=True, touch_count=False, ray_stats=False, tune: T.Tune | None = None,
             regrouped: bool = True) -> T.ForwardResult:
     """Forward trace of the camera's pixels; results by pixel, event-log columns by slot.
-    regrouped: with k-buffers of up to 16 events, pack the pixels still active after the
-    first gather rounds into full warps (ever_trace_forward_camera_regrouped; same results)."""
+    regrouped: with k-buffers of up to 16 events, run ever_trace_forward_camera_regrouped: same
+    results; rays that the default trace leaves to gather rounds run them in a kernel of their
+    own, and with gather rounds only (tune.traversal 2) the pixels still active after the first
+    rounds are packed into full warps."""
     device = scene.device
     R, S = camera.num_pixels, camera_slots(camera)
     jitter = _jitter(jitter, R, device)

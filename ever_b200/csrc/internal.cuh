@@ -60,6 +60,17 @@ cudaError_t scene_set_features(EverScene* sc, const float* feat, cudaStream_t st
 cudaError_t scene_refit(const float* mean, const float* scale, const float* quat, const float* density,
                         const float* feat, char* ws, const SceneLayout& L, EverScene* sc, cudaStream_t st);
 
+// Rays that the frustum kernel leaves to the gather rounds in their own kernel: all of a launch
+// whose rays come in no order (votes of sampled packets), and those of packets whose
+// leaf lists do not serve them, parked in the outputs, with their slots in the list.
+enum LeftWord { kLeftVotes, kLeftTaken, kLeftPackets, kLeftGroups, kLeftWords };
+struct LeftRays {
+  uint32_t* words;  // kLeftWords device words; null: no such kernel
+  int32_t* list;    // groups of 32 slots with such rays
+  uint32_t* masks;  // their bits, a word per group
+  uint32_t votes_min, packets_min;
+};
+
 struct FwdParams {
   const void* nodes;
   const void* records;
@@ -78,12 +89,7 @@ struct FwdParams {
   int stack_depth;  // traversal stack entries in use, <= kStackDepth (set from the tune)
   int lanes;        // frustum kernels: rays per packet, <= 32 (set by the launcher)
   const float* depth_hint;  // (R) nullable: per-ray guess of the stopping t (first frustum stage)
-  // A launch whose rays may come in no order: the sampled packets in which they do are counted
-  // in *votes, and from vote_min on the gather rounds trace the launch (taking packets from
-  // *taken) instead of the frustum kernel. Device words; null: no vote.
-  uint32_t* votes;
-  uint32_t* taken;
-  uint32_t vote_min;
+  LeftRays left;    // null words: every ray is finished in the frustum kernel
 };
 
 cudaError_t launch_forward(const FwdParams& P, int deg, const EverTune& tune, cudaStream_t st);
@@ -97,7 +103,7 @@ struct RegroupScratch {
   uint32_t* offsets;  // ceil(R/32) + 1: exclusive scan of a mask's popcounts
   int32_t* list1;     // R: slots of pass 1, in slot order
   int32_t* list2;     // R: slots of pass 2
-  uint32_t* count1;   // 1
+  uint32_t* count1;   // kLeftWords
   uint32_t* count2;   // 1
   int64_t split_min;  // a pass with fewer rays runs every remaining round (set by the launcher)
 };

@@ -92,7 +92,7 @@ int64_t regroup_workspace(int64_t R) {
   c.take((nw + 1) * 4);
   c.take(R * 4);
   c.take(R * 4);
-  c.take(4);
+  c.take(kLeftWords * 4);
   c.take(4);
   return c.offset;
 }
@@ -106,7 +106,7 @@ RegroupScratch regroup_scratch(char* ws, int64_t R) {
   W.offsets = reinterpret_cast<uint32_t*>(ws + c.take((nw + 1) * 4));
   W.list1 = reinterpret_cast<int32_t*>(ws + c.take(R * 4));
   W.list2 = reinterpret_cast<int32_t*>(ws + c.take(R * 4));
-  W.count1 = reinterpret_cast<uint32_t*>(ws + c.take(4));
+  W.count1 = reinterpret_cast<uint32_t*>(ws + c.take(kLeftWords * 4));
   W.count2 = reinterpret_cast<uint32_t*>(ws + c.take(4));
   W.split_min = 0;
   return W;
@@ -133,14 +133,15 @@ cudaError_t launch_forward_regrouped(const FwdParams& P0, const RegroupScratch& 
   if (P.R == 0) return cudaSuccess;
   const int block = tune.block > 0 ? tune.block : 128;
   // the frustum phase finishes nearly every ray of ordered packets in one launch: nothing to pack
-  // again; ray arrays in no order are for the rounds (a camera's tiles are always in order)
+  // again; the rays it leaves run the rounds in their own kernel
   if (P.frustum) {
     EverTune t = tune;
     t.traversal = 0;
     FwdParams F = P;
-    F.votes = W.count1;
-    F.taken = W.count2;
-    return cam ? launch_forward_camera(P, *cam, jitter, deg, t, st) : launch_forward(F, deg, t, st);
+    F.left.words = W.count1;
+    F.left.list = W.list1;
+    F.left.masks = W.mask0;
+    return cam ? launch_forward_camera(F, *cam, jitter, deg, t, st) : launch_forward(F, deg, t, st);
   }
   // splitting pays only while the next pass still fills the GPU several times over: four
   // times the resident lanes of the packet kernels (20 warps per SM)

@@ -308,6 +308,7 @@ struct TraceCtx {
   EverForwardOut out;
   int depth;           // traversal stack entries in use (<= kStackDepth)
   const float* depth_hint;  // (R) nullable: per-ray guess of the stopping t
+  LeftRays left;       // rays that the frustum phase leaves, for the rounds' own kernel
 };
 
 // One event of a ray's sorted sequence, integrated under the reference's round rules
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(256) k_trace_fwd_ray(const FwdParams P) {
   if (gi >= P.R) return;
   const int64_t r = P.ray_order ? int64_t(P.ray_order[gi]) : gi;
   const SceneRef sc = scene_of(P);
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint, P.left};
   const Ray ray = load_ray(P.rayo, P.rayd, r, P.tmin);
   const RaySlab sl = make_slab(ray);
   float B[16];
@@ -572,6 +573,13 @@ constexpr int kCandCap = kStageLeaves + 64;
 // wide packets of small views cut too long (batched views 4.4 -> 5.0 ms).
 constexpr int kMaxCuts = 16;
 constexpr int kMaxStages = 128;  // then the rounds take over
+// Passes over a stage's list, after which the stage ends where its slowest lane is and the next
+// lists half as many leaves (kShortList at least): where a ray is inside many ellipsoids at
+// once, each pass tests every leaf for the few events that a lane's buffer takes (262,144 rays
+// through 10,000 ellipsoids three times over 10.1 -> 7.3 ms; with 3 passes a dense uniform
+// scene 1.02 -> 1.14 ms, with 8 the first 7.8).
+constexpr int kMaxPasses = 5;
+constexpr int kShortList = 96;
 constexpr int kTileWords = 28;
 constexpr int kStateWords = 14;  // of a lane's integration state: State (13), the last event's id
 // Shared ints per warp: the walk's nodes with their entry bounds (before and after it, the
@@ -1014,7 +1022,7 @@ __device__ __noinline__ LeafList list_leaves(const Node* nodes, const Record* re
   float area;
   const PacketBounds P = packet_bounds(ray, make_slab(ray), mine, tile, lane, &area);
   const bool cull = area < INFINITY;
-  const int n = packet_leaves(nodes, recs, P, tile, cull, t_lo, &cap, cull ? limit : kStageLeaves, walk, cand, lane);
+  const int n = packet_leaves(nodes, recs, P, tile, cull, t_lo, &cap, cull || limit < kFirstLeaves ? limit : kStageLeaves, walk, cand, lane);
   if (n > 0) sort_keys(cand, n, lane);
   return LeafList{n, cap, area};
 }
@@ -1234,6 +1242,7 @@ __device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx
   const int first = L.iters;
   float t_done = 0.f;  // every event of this lane's ray before it has been taken
   float whole = INFINITY;  // tile area of the group a half was taken from
+  int limit = kFirstLeaves;
   unsigned todo = __ballot_sync(kFull, act), grp = pick_group(ray, todo, lane);
   if (grp == todo && no_order(ray, todo, lane)) return act;
 #pragma unroll 1
@@ -1248,21 +1257,19 @@ __device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx
       if (h > 0.f && 1.05f * h + 1e-3f < cap) cap = 1.05f * h + 1e-3f;
     }
     const LeafList list = list_leaves(sc.nodes, sc.recs, ray.o, ray.d, ray.apex, mine, t_lo, cap,
-                                      t_lo == 0.f ? kFirstLeaves : kStageLeaves, at, lane);
+                                      t_lo == 0.f ? min(limit, kFirstLeaves) : limit, at, lane);
     int nc = list.n;
     const bool cut = list.cap < cap;
     cap = list.cap;
     // half a group's lanes cover as much as all did: directions in no order, for the rounds
     if (list.area > 0.7f * whole) break;
     whole = INFINITY;
-    if (nc < 0) {  // does not fit: fewer rays at a time, or the rounds
-      if (__popc(grp) > 1 && list.area < INFINITY) {
-        whole = list.area;
-        grp = half_group(grp, lane);
-      } else {
-        todo &= ~grp;
-        grp = pick_group(ray, todo, lane);
-      }
+    // More leaves than the list holds reach over one t. Fewer rays at a time would hardly meet
+    // fewer of them (1,000 large ellipsoids among 50,000, 262,144 rays: halved down to single
+    // rays 157 ms, left to the rounds 32).
+    if (nc < 0) {
+      if (limit >= kFirstLeaves) break;
+      limit = kStageLeaves;
       continue;
     }
     // events from `end` on belong to the next stage
@@ -1274,7 +1281,7 @@ __device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx
     // events and takes those; the events from `over` (the smallest it dropped) on are
     // collected again by another pass.
     bool pending = mine;
-    int hits = 0;
+    int hits = 0, passes = 0;
 #pragma unroll 1
     do {
       uint64_t buf[FBUF];
@@ -1323,10 +1330,13 @@ __device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx
         }
       }
       pending = pending && act && over < end;
-    } while (__any_sync(kFull, pending));
+    } while (__any_sync(kFull, pending) && ++passes < kMaxPasses);
+    const bool ended = __any_sync(kFull, pending);
+    if (ended) limit = max(kShortList, limit / 2);
+    else if (limit >= kFirstLeaves) limit = kStageLeaves;
     if (mine) {
-      t_done = cap;
-      if (cap >= cap_all) act = false;
+      t_done = pending ? fminf(fmaxf(t_lo, key_t(L.lower)), cap_all) : cap;  // exits may lie beyond tmax
+      if (!pending && cap >= cap_all) act = false;
     }
     const unsigned left = __ballot_sync(kFull, act);
     // a list that had to be cut short and that fewer than one lane in 32 met on average: the
@@ -1334,10 +1344,6 @@ __device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx
     const bool wide = __reduce_add_sync(kFull, hits) * 32 < nc * __popc(grp);
     todo &= left;
     grp &= left;
-    if (cut && !(list.area < INFINITY)) {  // no apex to halve the directions around: the rounds
-      todo &= ~grp;
-      grp = 0;
-    }
     if (!grp) {
       grp = pick_group(ray, todo, lane);
     } else if (cut && wide && __popc(grp) > 1) {
@@ -1350,48 +1356,6 @@ __device__ __forceinline__ bool frustum_phase(const SceneRef& sc, const TraceCtx
   if (L.iters > first) L.last_dirac = event_dirac<DEG>(sc, B, bs, __float_as_uint(q.st[32 * 13 + lane]));
   __syncwarp();
   return act;
-}
-
-// The rounds that finish what the frustum phase leaves: rarely anything, so they are a call
-// (inlined, they would cost the whole kernel registers), with its arguments in local memory.
-struct RoundsCall {
-  SceneRef sc;
-  TraceCtx C;
-  Ray ray;
-  const float* B;
-  int bs, lane;
-  int64_t slot;
-  int* wstack;
-  bool act;
-  RayLoop L;
-};
-template <int KBUF, int DEG>
-__device__ __noinline__ void rounds_call(RoundsCall* a) {
-  RayLoop L = a->L;
-  run_rounds<KBUF, DEG>(a->sc, a->C, a->ray, a->B, a->bs, a->slot, a->wstack, a->lane, a->act, L, INT_MAX);
-  a->L = L;
-}
-
-// One warp traces one packet of up to 32 rays against one scene (lanes with valid=false
-// only take part in the warp-wide votes). FRUSTUM: the frustum phase, else rounds only.
-template <int KBUF, int DEG, bool FRUSTUM>
-__device__ __forceinline__ void trace_packet(const SceneRef& sc, const TraceCtx& C, const Ray& ray, int64_t r,
-                                             bool valid, int64_t slot, int* wstack, float* B, int bs, int lane) {
-  store_basis<DEG>(ray, B, bs);
-  RayLoop L = start_ray<DEG>(sc, ray, valid, wstack, C.depth, B, bs, lane);
-  bool act = valid && C.max_iters > 0 && sc.N > 0;
-  if (FRUSTUM) {
-    act = frustum_phase<KBUF, DEG>(sc, C, ray, B, bs, slot, r, int(threadIdx.x >> 5) * kWarpInts, lane, act, L);
-    if (__any_sync(kFull, act)) {
-      RoundsCall a{sc, C, ray, B, bs, lane, slot, wstack, act, L};
-      rounds_call<KBUF, DEG>(&a);
-      L = a.L;
-    }
-  } else {
-    run_rounds<KBUF, DEG>(sc, C, ray, B, bs, slot, wstack, lane, act, L, INT_MAX);
-  }
-  if (valid) write_outputs(C.out, r, L.s, L.last_dirac, L.iters, L.status);
-  __syncwarp();
 }
 
 // A ray that needs more rounds parks its loop state in its own output rows: `states` in
@@ -1429,6 +1393,80 @@ __device__ __forceinline__ RayLoop resume_ray(const EverForwardOut& out, int64_t
   return L;
 }
 
+// Rounds that a packet runs itself on the rays that the frustum phase leaves it. Inside this
+// kernel they have 16 warps per SM and the L1 that the lists leave, in their own 20 and nearly
+// all of it; but a few rays there would run alone. So the first packets of a launch (as many as
+// are resident) run two rounds, which is all that most such rays need (100,000 uniform
+// ellipsoids all around, 262,144 rays: 2.8 ms, with every packet left at once 3.5); what
+// they leave, and every later packet's rays, are the other kernel's (1,000 large ellipsoids
+// among 50,000: 34 ms, with all rounds here 49).
+constexpr int kRoundsHere = 2;
+__device__ __forceinline__ int rounds_here(const LeftRays& left, int lane) {
+  if (!left.words) return INT_MAX;
+  uint32_t n = 0;
+  if (lane == 0) n = atomicAdd(left.words + kLeftPackets, 1u);
+  return __shfl_sync(kFull, n, 0) < left.packets_min ? kRoundsHere : 0;
+}
+
+// Lists the rays m of the packet of slots [first, first + 32).
+__device__ __forceinline__ void leave_rays(const LeftRays& left, unsigned m, int64_t first, int lane) {
+  if (lane != 0) return;
+  left.masks[first >> 5] = m;
+  left.list[atomicAdd(left.words + kLeftGroups, 1u)] = int32_t(first >> 5);
+}
+
+// The rounds that finish what the frustum phase leaves: rarely anything, so they are a call
+// (inlined, they would cost the whole kernel registers), with its arguments in local memory.
+struct RoundsCall {
+  SceneRef sc;
+  TraceCtx C;
+  Ray ray;
+  const float* B;
+  int bs, lane;
+  int64_t slot;
+  int* wstack;
+  bool act;
+  RayLoop L;
+  int rounds;
+};
+template <int KBUF, int DEG>
+__device__ __noinline__ void rounds_call(RoundsCall* a) {
+  RayLoop L = a->L;
+  a->act = run_rounds<KBUF, DEG>(a->sc, a->C, a->ray, a->B, a->bs, a->slot, a->wstack, a->lane, a->act, L, a->rounds);
+  a->L = L;
+}
+
+// One warp traces one packet of up to 32 rays against one scene (lanes with valid=false
+// only take part in the warp-wide votes). FRUSTUM: the frustum phase, else rounds only.
+template <int KBUF, int DEG, bool FRUSTUM>
+__device__ __forceinline__ void trace_packet(const SceneRef& sc, const TraceCtx& C, const Ray& ray, int64_t r,
+                                             bool valid, int64_t slot, int* wstack, float* B, int bs, int lane) {
+  store_basis<DEG>(ray, B, bs);
+  RayLoop L = start_ray<DEG>(sc, ray, valid, wstack, C.depth, B, bs, lane);
+  bool act = valid && C.max_iters > 0 && sc.N > 0;
+  if (FRUSTUM) {
+    act = frustum_phase<KBUF, DEG>(sc, C, ray, B, bs, slot, r, int(threadIdx.x >> 5) * kWarpInts, lane, act, L);
+    if (__any_sync(kFull, act)) {
+      const int rounds = rounds_here(C.left, lane);
+      if (rounds > 0) {
+        RoundsCall a{sc, C, ray, B, bs, lane, slot, wstack, act, L, rounds};
+        rounds_call<KBUF, DEG>(&a);
+        L = a.L;
+        act = a.act;
+      }
+      if (const unsigned m = __ballot_sync(kFull, act)) {
+        leave_rays(C.left, m, slot - lane, lane);
+        if (act) park_ray(C.out, r, L);
+        valid = valid && !act;  // the outputs of those are the rounds' to write
+      }
+    }
+  } else {
+    run_rounds<KBUF, DEG>(sc, C, ray, B, bs, slot, wstack, lane, act, L, INT_MAX);
+  }
+  if (valid) write_outputs(C.out, r, L.s, L.last_dirac, L.iters, L.status);
+  __syncwarp();
+}
+
 // Resident blocks per SM that the register budget of the packet kernels targets: 16 warps
 // (128 registers) with the frustum phase, which is bound by instructions and not by latency
 // (3.6 ms at 1M ellipsoids / 1080p; 20 warps: 4.0 ms, with spills); 20 warps (96
@@ -1441,14 +1479,14 @@ struct FwdMinBlocks {
 template <int KBUF, int DEG, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK>::value) k_trace_fwd_packet(const FwdParams P) {
   extern __shared__ int smem[];
-  if (P.votes && __ldg(P.votes) >= P.vote_min) return;  // the rounds trace this launch
+  if (P.left.words && __ldg(P.left.words + kLeftVotes) >= P.left.votes_min) return;  // the rounds trace this launch
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int* wstack = smem + warp * kWarpInts;  // traversal stack, and the frustum phase's lists over it
   float* B = reinterpret_cast<float*>(smem + (blockDim.x / 32) * kWarpInts) + tid;  // B[k * blockDim.x]
   const int64_t gi = (int64_t(blockIdx.x) * (blockDim.x / 32) + warp) * P.lanes + lane;
   const bool valid = lane < P.lanes && gi < P.R;  // every lane stays for the warp-wide ballots
   const int64_t r = valid ? (P.ray_order ? int64_t(P.ray_order[gi]) : gi) : 0;
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint, P.left};
   const Ray ray = load_ray(P.rayo, P.rayd, r, P.tmin);
   trace_packet<KBUF, DEG, true>(scene_of(P), C, ray, r, valid, gi, wstack, B, blockDim.x, lane);
 }
@@ -1492,7 +1530,7 @@ __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK, false>::value)
   }
   if (!valid) r = 0;
   const SceneRef sc = scene_of(P);
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint, P.left};
   Ray ray;
   if (CAM) {
     float3 ro, rd;
@@ -1550,35 +1588,56 @@ __global__ void __launch_bounds__(1024) k_order_vote(const FwdParams P, uint32_t
   }
   if (lane == 0 && n) atomicAdd(&votes, n);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    *P.votes = votes;
-    *P.taken = 0;
-  }
+  if (threadIdx.x < kLeftWords) P.left.words[threadIdx.x] = threadIdx.x == kLeftVotes ? votes : 0u;
 }
 
-// The rounds of a launch in no order. Persistent (an empty launch of one block per packet takes
-// 10 us at full HD): warps take packets from a device counter.
-constexpr int kUnorderedBlock = 128;
-template <int KBUF, int DEG>
-__global__ void __launch_bounds__(kUnorderedBlock, FwdMinBlocks<kUnorderedBlock, false>::value)
-    k_trace_fwd_unordered(const FwdParams P) {
+// The rounds of a launch in no order, or of the rays that the frustum kernel has parked in the
+// list. Persistent (an empty launch of one block per packet takes 10 us at full HD): warps take
+// 32 slots at a time from a device counter.
+constexpr int kLeftBlock = 128;
+template <int KBUF, int DEG, bool CAM>
+__global__ void __launch_bounds__(kLeftBlock, FwdMinBlocks<kLeftBlock, false>::value)
+    k_trace_fwd_left(const FwdParams P, const PassCamera Q) {
   extern __shared__ int smem[];
-  if (__ldg(P.votes) < P.vote_min) return;  // the frustum kernel has traced this launch
+  const bool all = !CAM && __ldg(P.left.words + kLeftVotes) >= P.left.votes_min;
+  const int64_t n = all ? P.R : 32 * int64_t(__ldg(P.left.words + kLeftGroups));
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int* wstack = smem + warp * kStackDepth;
-  float* B = reinterpret_cast<float*>(smem + (kUnorderedBlock / 32) * kStackDepth) + tid;
+  float* B = reinterpret_cast<float*>(smem + (kLeftBlock / 32) * kStackDepth) + tid;
   const SceneRef sc = scene_of(P);
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
-  for (;;) {
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint, {}};
+  while (n > 0) {
     uint32_t packet = 0;
-    if (lane == 0) packet = atomicAdd(P.taken, 1u);
+    if (lane == 0) packet = atomicAdd(P.left.words + kLeftTaken, 1u);
     packet = __shfl_sync(kFull, packet, 0);
     const int64_t gi = int64_t(packet) * 32 + lane;
-    if (int64_t(packet) * 32 >= P.R) break;
-    const bool valid = gi < P.R;
-    const int64_t r = valid ? (P.ray_order ? int64_t(P.ray_order[gi]) : gi) : 0;
-    const Ray ray = load_ray(P.rayo, P.rayd, r, P.tmin);
-    trace_packet<KBUF, DEG, false>(sc, C, ray, r, valid, gi, wstack, B, kUnorderedBlock, lane);
+    if (int64_t(packet) * 32 >= n) break;
+    const int32_t group = all ? int32_t(packet) : P.left.list[packet];
+    const bool valid = all ? gi < n : P.left.masks[group] >> lane & 1u;
+    const int64_t slot = valid ? 32 * int64_t(group) + lane : 0;
+    int64_t r = slot;
+    if (CAM) r = valid ? camera_slot_pixel(Q.cam, slot) : 0;
+    else if (P.ray_order) r = valid ? int64_t(P.ray_order[slot]) : 0;
+    Ray ray;
+    if (CAM) {
+      float3 ro, rd;
+      camera_ray(Q.cam, Q.jitter, r, ro, rd);
+      ray = make_ray(ro, rd, P.tmin);
+    } else {
+      ray = load_ray(P.rayo, P.rayd, r, P.tmin);
+    }
+    store_basis<DEG>(ray, B, kLeftBlock);
+    RayLoop L;
+    bool act = valid;
+    if (all) {
+      L = start_ray<DEG>(sc, ray, valid, wstack, C.depth, B, kLeftBlock, lane);
+      act = valid && C.max_iters > 0 && sc.N > 0;
+    } else if (valid) {
+      L = resume_ray(P.out, r);
+    }
+    run_rounds<KBUF, DEG>(sc, C, ray, B, kLeftBlock, slot, wstack, lane, act, L, INT_MAX);
+    if (valid) write_outputs(C.out, r, L.s, L.last_dirac, L.iters, L.status);
+    __syncwarp();
   }
 }
 
@@ -1596,7 +1655,7 @@ __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK>::value)
   const int64_t gi = (int64_t(blockIdx.x) * (blockDim.x / 32) + warp) * P.lanes + lane;
   const int64_t p = lane < P.lanes && gi < num_slots ? camera_slot_pixel(cam, gi) : -1;
   const bool valid = p >= 0;
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint};
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, P.depth_hint, P.left};
   float3 ro, rd;
   camera_ray(cam, jitter, valid ? p : 0, ro, rd);
   const Ray ray = make_ray(ro, rd, P.tmin);
@@ -1613,7 +1672,7 @@ __global__ void __launch_bounds__(BLOCK, FwdMinBlocks<BLOCK, FRUSTUM>::value)
   constexpr int kInts = FRUSTUM ? kWarpInts : kStackDepth;  // traversal stack, and the frustum phase's lists over it
   int* wstack = smem + warp * kInts;
   float* B = reinterpret_cast<float*>(smem + (blockDim.x / 32) * kInts) + tid;
-  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, nullptr};
+  const TraceCtx C{P.tmin, P.tmax, P.max_iters, P.out, P.stack_depth, nullptr, {}};
   const int lanes = FRUSTUM ? P.lanes : 32;  // a divisor of 32: a packet never mixes views
   const int64_t num_packets = P.num_slots / lanes;
   for (;;) {
@@ -1661,25 +1720,32 @@ inline int packet_lanes(int64_t rays) {
   return lanes;
 }
 
-// The vote of a launch of full packets. Narrow packets (launches that leave warps idle) have
-// none: theirs is the frustum kernel, and two more launches would cost them (2 us each).
-inline cudaError_t vote_begin(FwdParams& P, cudaStream_t st) {
-  const uint32_t packets = uint32_t(std::min<int64_t>(P.R / 32, kVotePackets));
-  if (P.lanes < 32 || packets == 0) P.votes = nullptr;
-  if (!P.votes) return cudaSuccess;
-  P.vote_min = packets / 2 + 1;
+// Before the frustum kernel: the vote of a launch of full packets (it clears the words), or the
+// words cleared.
+inline cudaError_t left_begin(FwdParams& P, int64_t slots, bool cam, cudaStream_t st) {
+  const uint32_t packets = uint32_t(std::min<int64_t>(slots / 32, kVotePackets));
+  if (P.lanes < 32 || packets == 0) P.left.words = nullptr;
+  if (!P.left.words) return cudaSuccess;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  P.left.packets_min = uint32_t(16 * sms);  // the resident warps
+  if (cam) {
+    P.left.votes_min = UINT32_MAX;
+    return cudaMemsetAsync(P.left.words, 0, kLeftWords * sizeof(uint32_t), st);
+  }
+  P.left.votes_min = packets / 2 + 1;
   k_order_vote<<<1, 1024, 0, st>>>(P, packets);
   return cudaGetLastError();
 }
-template <int KBUF, int DEG>
-cudaError_t vote_finish(const FwdParams& P, cudaStream_t st) {
-  if (!P.votes) return cudaGetLastError();
+template <int KBUF, int DEG, bool CAM>
+cudaError_t left_finish(const FwdParams& P, const PassCamera& Q, cudaStream_t st) {
+  if (!P.left.words) return cudaGetLastError();
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem = packet_smem<DEG>(kUnorderedBlock, false);
-  if (cudaError_t e_ = prepare(k_trace_fwd_unordered<KBUF, DEG>, smem)) return e_;
-  k_trace_fwd_unordered<KBUF, DEG>
-      <<<sms * FwdMinBlocks<kUnorderedBlock, false>::value, kUnorderedBlock, smem, st>>>(P);
+  const size_t smem = packet_smem<DEG>(kLeftBlock, false);
+  if (cudaError_t e_ = prepare(k_trace_fwd_left<KBUF, DEG, CAM>, smem)) return e_;
+  k_trace_fwd_left<KBUF, DEG, CAM>
+      <<<sms * FwdMinBlocks<kLeftBlock, false>::value, kLeftBlock, smem, st>>>(P, Q);
   return cudaGetLastError();
 }
 
@@ -1716,7 +1782,7 @@ cudaError_t launch_t(const FwdParams& P0, int block, int traversal, cudaStream_t
   } else if (traversal == 2) {
     return launch_rounds<KBUF, DEG, false>(P, PassCamera{}, block, st);
   } else {
-    if (cudaError_t e_ = vote_begin(P, st)) return e_;
+    if (cudaError_t e_ = left_begin(P, P.R, false, st)) return e_;
     const size_t smem = packet_smem<DEG>(block);
     switch (block) {
       case 64: {
@@ -1735,7 +1801,7 @@ cudaError_t launch_t(const FwdParams& P0, int block, int traversal, cudaStream_t
         break;
       }
     }
-    return vote_finish<KBUF, DEG>(P, st);
+    return left_finish<KBUF, DEG, false>(P, PassCamera{}, st);
   }
   return cudaGetLastError();
 }
@@ -1809,6 +1875,7 @@ cudaError_t launch_camera_t(const FwdParams& P0, const CameraParams& cam, const 
   FwdParams P = P0;
   P.lanes = packet_lanes(num_slots);
   const unsigned grid = unsigned((num_slots + P.lanes * (block / 32) - 1) / (P.lanes * (block / 32)));
+  if (cudaError_t e_ = left_begin(P, num_slots, true, st)) return e_;
   const size_t smem = packet_smem<DEG>(block);
   switch (block) {
     case 64: {
@@ -1827,7 +1894,7 @@ cudaError_t launch_camera_t(const FwdParams& P0, const CameraParams& cam, const 
       break;
     }
   }
-  return cudaGetLastError();
+  return left_finish<KBUF, DEG, true>(P, PassCamera{cam, jitter, num_slots}, st);
 }
 
 template <int KBUF>

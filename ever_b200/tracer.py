@@ -165,8 +165,9 @@ def forward(scene: Scene, rayo, rayd, tmin=0.0, tmax=1000.0, max_iters=500, sh_d
             workspace: torch.Tensor | None = None, depth_hint: torch.Tensor | None = None) -> ForwardResult:
     """regrouped: with warp packets (tune.traversal 0 or 2) and k-buffers of up to 16 events, run
     ever_trace_forward_regrouped: same results; with traversal 2 the rays that need more gather
-    rounds are packed into full warps between passes, with traversal 0 a launch whose rays come
-    in no order runs the rounds in a kernel of their own. workspace: optional uint8 scratch of
+    rounds are packed into full warps between passes, with traversal 0 the rays that are left to
+    gather rounds (all of a launch in no order, those that lists of leaves do not serve) run them
+    in a kernel of their own. workspace: optional uint8 scratch of
     ever_trace_forward_workspace_bytes(R)."""
     device = scene.device
     _check_tensor("ray_origins", rayo, device, 3)

@@ -168,9 +168,10 @@ size_t ever_trace_forward_workspace_bytes(int64_t num_rays);
 /* ever_trace_forward, same arguments and the same results bit for bit, for warp-packet
  * traversal. With gather rounds only (traversal 2) the rays that need more rounds are packed
  * into full warps in launch order after each of the first two, so warps stop running with
- * most of their lanes idle. With the frustum phase (traversal 0) nothing is packed; a launch that
- * fills the GPU first looks whether its rays come in any order (64 of its packets), and if
- * not traces them with gather rounds in a kernel of their own. Traversal 1: as 2 where a
+ * most of their lanes idle. With the frustum phase (traversal 0) a launch of full packets (one
+ * that fills the GPU) runs gather rounds in a kernel of their own: for all its rays, if 64 of its
+ * packets show that they come in no order, and for those that lists of leaves do not serve.
+ * Traversal 1: as 2 where a
  * launch is large enough to split (regroup_min), else as 0. Rays between passes keep their
  * loop state in out->states and out->last_dirac, which are therefore required. R < 2^31.
  * No counterpart in the reference (OptiX runs one thread per ray to the end). */
