@@ -117,8 +117,9 @@ template <int KBUF>
 __device__ void gather_ray(const Node* __restrict__ nodes, const Record* __restrict__ recs, const Ray& ray,
                            const RaySlab& sl, uint64_t lower, float s16, float tmax, uint64_t (&buf)[KBUF],
                            int* st_node, float* st_t, int stride, int depth, uint32_t& status) {
-  const float lo_t = fmaxf(lower ? key_t(lower) : 0.f, s16);
   const float cap = fminf(tmax, kSentinel);
+  // The last event may be an exit beyond tmax; others like it are still to be found at tmax.
+  const float lo_t = fminf(fmaxf(lower ? key_t(lower) : 0.f, s16), cap);
   int sp = 0;
   int node = 0;
   for (;;) {
@@ -166,8 +167,8 @@ template <int KBUF>
 __device__ void gather_packet(const Node* __restrict__ nodes, const Record* __restrict__ recs, const Ray& ray,
                               const RaySlab& sl, bool act, uint64_t lower, float s16, float tmax,
                               uint64_t (&buf)[KBUF], int* wstack, int lane, int depth, uint32_t& status) {
-  const float lo_t = fmaxf(lower ? key_t(lower) : 0.f, s16);
   const float cap = fminf(tmax, kSentinel);
+  const float lo_t = fminf(fmaxf(lower ? key_t(lower) : 0.f, s16), cap);  // as in gather_ray
   int sp = 0;
   int node = 0;
   for (;;) {
