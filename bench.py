@@ -708,7 +708,7 @@ def main():
     # DRAM bytes per call (dram__bytes_read.sum + dram__bytes_write.sum over the call's trace
     # kernels) from one single-pass ncu capture of `bench.py --once` on this default workload
     # (1M ellipsoids, 1920x1080): forward = k_trace_fwd_packet, backward = k_trace_bwd
-    measured_traffic = {"fwd": 274_770_000 + 405_020_000, "bwd": 1_160_140_000 + 141_560_000}
+    measured_traffic = {"fwd": 273_570_000 + 406_240_000, "bwd": 1_158_070_000 + 140_350_000}
     default_workload = args.prims == 1_000_000 and args.width == 1920 and args.height == 1080
     roofline = {"bound": "hbm",
                 "kernel": "k_trace_bwd" if dom == "bwd" else "k_trace_fwd_packet",
@@ -716,7 +716,7 @@ def main():
                 "peak_kind": peak_kind, "traffic": measured_traffic[dom] if default_workload else None,
                 "algorithmic_bytes": b_dom,
                 "note": "issue-bound tree walk and event integration, not HBM-bound"
-                        + (": the forward issues on 53% of cycles (ALU pipe 41%) while DRAM moves under 2% of its "
+                        + (": the forward issues on 54% of cycles (ALU pipe 41%) while DRAM moves under 2% of its "
                            "peak" if default_workload else "")}
 
     line = {

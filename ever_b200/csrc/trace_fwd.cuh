@@ -1,16 +1,16 @@
 // Forward trace kernels (included by trace_fwd_k{8,16,32}.cu, one k-buffer size per
 // translation unit so the instantiations compile in parallel).
 //
-// LBVH traversal that gathers each ray's next KBUF entry/exit events into
-// a sorted register buffer, then integrates them in order (update() with SH colour
-// evaluated along the ray), round after round.
-//
-// Two traversals share the same gather/consume semantics:
-//  - packet (default): the 32 rays of a warp walk ONE node sequence together. Each
-//    lane tests its own ray against the node's two child boxes, __ballot_sync decides
-//    where the warp goes, and a per-warp stack lives in shared memory. Node fetches
-//    are warp-uniform (one broadcast load) and the control flow never diverges.
-//  - per-ray: each thread walks the tree alone (stack in shared memory per thread).
+// Each ray's entry/exit events are integrated in order of t (update() with SH colour
+// evaluated along the ray). Three traversals find them, with the same results:
+//  - frustum phase (traversal 0, the default): the warp lists the leaves that its packet of
+//    up to 32 rays can meet, and each lane takes its events from that list (below);
+//  - gather rounds of packets (2, and what the frustum phase leaves): each ray's next KBUF
+//    events go into a sorted register buffer and are then integrated, round after round. The
+//    rays of a warp walk ONE node sequence together: each lane tests its own ray against
+//    the node's two child boxes, __ballot_sync decides where the warp goes, and a per-warp
+//    stack lives in shared memory. Node fetches are warp-uniform (one broadcast load);
+//  - gather rounds per ray (1): each thread walks the tree alone (stack in shared memory).
 //
 // Reference: raygen loop splinetracers/fast_ellipsoid_splinetracer/slang/shaders.slang:171-235,
 // intersection program :84-107 and any-hit k-buffer :117-164. Our rounds gather
@@ -536,7 +536,7 @@ __device__ __forceinline__ bool run_rounds(const SceneRef& sc, const TraceCtx& C
 }
 
 // ---- packet frustum phase ----
-// Bound by issued instructions (55% of the issue slots busy, ALU pipe 42%, DRAM 1%), so the
+// Bound by issued instructions (54% of the issue slots busy, ALU pipe 41%, DRAM 2%), so the
 // phase is cut into steps that each keep the lanes busy:
 //  - list_leaves: the warp bounds its rays by intervals (origins, inverse directions), walks
 //    the BVH with one child box per lane and lists the leaves whose box some ray can meet;
@@ -552,7 +552,8 @@ __device__ __forceinline__ bool run_rounds(const SceneRef& sc, const TraceCtx& C
 // leaves of the whole t range do not fit, the phase goes on in stages over t. At 1M
 // ellipsoids / 1080p the forward's kernels took 6.26 ms before (one walk over whole nodes,
 // no cone test, integration where an event became final, a second pass of stack rounds for
-// overflowing packets) and take 3.5 ms; a packet issues 33k instructions, 66k before.
+// overflowing packets) and take 3.6 ms; a packet issues 37k instructions, 66k before. The
+// sweeps below were taken when it was 3.5 ms, by event times within one run.
 // Rays in no order (no_order) have no list in common and go to the rounds at once.
 // Events a lane holds in the frustum phase: more cost registers and compares, fewer cost the
 // lanes that run out another pass over the list (kernel time at 1M ellipsoids / 1080p and for
@@ -1410,7 +1411,7 @@ __device__ __forceinline__ RayLoop resume_ray(const EverForwardOut& out, int64_t
 // are resident) run two rounds, which is all that most such rays need (100,000 uniform
 // ellipsoids all around, 262,144 rays: 2.8 ms, with every packet left at once 3.5); what
 // they leave, and every later packet's rays, are the other kernel's (1,000 large ellipsoids
-// among 50,000: 34 ms, with all rounds here 49).
+// among 50,000: 37 ms, with all rounds here 50).
 constexpr int kRoundsHere = 2;
 __device__ __forceinline__ int rounds_here(const LeftRays& left, int lane) {
   if (!left.words) return INT_MAX;
@@ -1480,7 +1481,7 @@ __device__ __forceinline__ void trace_packet(const SceneRef& sc, const TraceCtx&
 
 // Resident blocks per SM that the register budget of the packet kernels targets: 16 warps
 // (128 registers) with the frustum phase, which is bound by instructions and not by latency
-// (3.6 ms at 1M ellipsoids / 1080p; 20 warps: 4.0 ms, with spills); 20 warps (96
+// (20 warps, with spills: 4.0 against 3.6 ms at 1M ellipsoids / 1080p); 20 warps (96
 // registers) for the rounds, whose traversal is latency-bound.
 template <int BLOCK, bool FRUSTUM = true>
 struct FwdMinBlocks {
