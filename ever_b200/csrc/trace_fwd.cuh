@@ -1736,7 +1736,7 @@ inline int packet_lanes(int64_t rays) {
 // words cleared.
 inline cudaError_t left_begin(FwdParams& P, int64_t slots, bool cam, cudaStream_t st) {
   const uint32_t packets = uint32_t(std::min<int64_t>(slots / 32, kVotePackets));
-  if (P.lanes < 32 || packets == 0) P.left.words = nullptr;
+  if (P.lanes < 32 || packets == 0 || P.max_iters <= 0) P.left.words = nullptr;  // no iterations: no rounds
   if (!P.left.words) return cudaSuccess;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -114,3 +114,17 @@ def test_many_leaves_over_one_t_cost_what_the_rounds_cost(rays):
             best[m] = min(best[m], a.elapsed_time(b))
     print(f"{rays}: default {best[0]:.2f} ms, rounds {best[2]:.2f} ms")
     assert best[0] < 2.0 * best[2], best
+
+
+@pytest.mark.parametrize("max_iters,kernels", [(0, 1), (1, 3)])
+def test_no_iterations_need_no_second_kernel(max_iters, kernels):
+    # the start density alone (sp.Forward's initial_drgb): neither vote nor rounds
+    scene = _scene("large", 20_000)
+    ro, rd = _rays("view", 256, 256)
+    T.forward(scene, ro, rd, 0.0, 1000.0, max_iters)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        T.forward(scene, ro, rd, 0.0, 1000.0, max_iters)
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if "k_order_vote" in e.name or "k_trace_fwd" in e.name]
+    assert len(names) == kernels, names
